@@ -22,6 +22,7 @@
 
 #include <algorithm>
 
+#include "bulk.cuh"
 #include "common.cuh"
 #include "dispatch.cuh"
 #include "lookback.cuh"
@@ -483,6 +484,496 @@ __global__ void __launch_bounds__(kThreads, 4)
   }
 }
 
+// ------------------------------------------------- warp-window kernels --
+//
+// Plain columns of 4- and 8-byte elements whose order is that of unsigned
+// words after a bijection (integers under any predicate, floats in the total
+// order), and, for the set operations, floats under LESS / GREATER (-0 mapped
+// to +0, which tie).  What bounded the thread-serial kernels below was
+// instruction issue (merge 2 x 2^25 u32: 88% of issue slots, 103 warp
+// instructions per 32 outputs; set_intersection 250): each thread searched
+// its own split in shared memory and then took one dependent step per output.
+// Here a warp takes a whole window of both inputs per step: the items of
+// window A and of window B reversed, compared lane by lane, give the split of
+// the next 32 x R outputs with one ballot per register (the merge-path
+// predicate is monotone along the diagonal), so there is no search per
+// thread and every shared-memory access is to consecutive words.
+
+// Order- and equivalence-preserving map to unsigned words.  ENC: 0 integers
+// (raw ^ flip), 1 floats under LESS / GREATER, 2 floats in the total order;
+// `flip` holds the sign flip of signed integers and the inversion of GREATER.
+template <class U, int ENC>
+__device__ __forceinline__ U ord_of(U raw, U flip) {
+  if constexpr (ENC == 0) {
+    return raw ^ flip;
+  } else {
+    constexpr U sign = (U)1 << (sizeof(U) * 8 - 1);
+    if constexpr (ENC == 1) {
+      if (raw == sign) raw = 0;
+    }
+    return enc_bits<U, kEncFloat>(raw) ^ flip;
+  }
+}
+// The raw bits of an ordered word (ENC 0 and 2 are bijections).
+template <class U, int ENC>
+__device__ __forceinline__ U ord_to_raw(U u, U flip) {
+  u ^= flip;
+  if constexpr (ENC == 2) {
+    constexpr U sign = (U)1 << (sizeof(U) * 8 - 1);
+    return (u & sign) ? (U)(u ^ sign) : (U)~u;
+  }
+  return u;
+}
+
+// The merge-path split of every tile boundary by groups of eight lanes: nine
+// sub-ranges per round, so a 27-step binary search becomes nine rounds of
+// independent loads (the searches' latency, not their traffic, is what the
+// tile kernel waits for).  Boundaries past the logical end are not computed.
+constexpr int kSplitLanes = 8;
+
+template <class U, int ENC>
+__global__ void __launch_bounds__(kThreads)
+    window_splits_kernel(Src L, Src R, uint32_t tile_items, uint64_t tiles, U flip,
+                         uint32_t* __restrict__ splits) {
+  const uint64_t nl = src_len(L), nr = src_len(R), n = nl + nr;
+  const U* l = (const U*)L.data;
+  const U* r = (const U*)R.data;
+  const int lane = threadIdx.x & 31, sub = lane & (kSplitLanes - 1);
+  const int shift = lane & ~(kSplitLanes - 1);
+  const uint64_t b =
+      (blockIdx.x * (uint64_t)kThreads + threadIdx.x) / kSplitLanes;
+  // (a boundary of the last, partial tile is still wanted: b * tile < n + tile)
+  const bool on = b <= tiles && b * tile_items < n + tile_items;
+  const uint64_t d = on ? min(b * tile_items, n) : 0;
+  uint64_t lo = d > nr ? d - nr : 0, hi = d < nl ? d : nl;
+  while (__any_sync(kFull, lo < hi)) {
+    const uint64_t step = (hi - lo + kSplitLanes) / (kSplitLanes + 1);
+    const uint64_t mid = lo + (uint64_t)(sub + 1) * step - 1;
+    bool before = false;  // the split lies after mid
+    if (lo < hi && mid < hi)
+      before = ord_of<U, ENC>(l[mid], flip) <= ord_of<U, ENC>(r[d - 1 - mid], flip);
+    const uint32_t m = (__ballot_sync(kFull, before) >> shift) & ((1u << kSplitLanes) - 1u);
+    if (lo < hi) {
+      lo += (uint64_t)__popc(m) * step;
+      if (m != (1u << kSplitLanes) - 1u) hi = min(hi, lo + step - 1);
+    }
+  }
+  if (on && sub == 0) splits[b] = (uint32_t)lo;
+}
+
+// The slices of one tile in shared memory: left items at [a_off, a_off + la),
+// right items at [b_off, b_off + lb) of `buf`.
+struct TileSlices {
+  uint32_t i0, j0;  // global index of the first left / right item
+  int la, lb, a_off, b_off;
+};
+
+template <class U>
+__device__ __forceinline__ TileSlices tile_slices(uint64_t d0, uint64_t d1, uint32_t s0,
+                                                  uint32_t s1) {
+  constexpr int V = 16 / (int)sizeof(U);
+  const int total = (int)(d1 - d0);
+  TileSlices t;
+  t.i0 = s0;
+  t.j0 = (uint32_t)(d0 - s0);
+  // (unsorted inputs can give splits that go back: still in bounds)
+  t.la = s1 <= s0 ? 0 : (int)min(s1 - s0, (uint32_t)total);
+  t.lb = total - t.la;
+  t.a_off = (int)(t.i0 % V);
+  t.b_off = (t.a_off + t.la + V - 1) / V * V + (int)(t.j0 % V);
+  return t;
+}
+
+// Bulk-copies src[g0, g0 + len) to buf + off (off % V == g0 % V): whole
+// 16-byte vectors inside the column by one cp.async.bulk issued by thread 0,
+// whose bytes are returned for the barrier; the last items of a column whose
+// length is no multiple of a vector are copied by the calling threads.
+template <class U>
+__device__ __forceinline__ uint32_t slice_bytes(uint32_t g0, int len, uint64_t n) {
+  constexpr uint64_t V = 16 / sizeof(U);
+  if (len == 0) return 0;
+  const uint64_t lo = g0 / V * V;
+  const uint64_t hi = min(((uint64_t)g0 + len + V - 1) / V * V, n / V * V);
+  return hi > lo ? (uint32_t)((hi - lo) * sizeof(U)) : 0u;
+}
+template <class U>
+__device__ __forceinline__ void slice_load(U* buf, int off, const U* src, uint32_t g0,
+                                           uint32_t bytes, uint64_t* bar) {
+  constexpr uint64_t V = 16 / sizeof(U);
+  if (bytes) bulk_load(buf + off - (int)(g0 % V), src + g0 / V * V, bytes, bar);
+}
+template <class U>
+__device__ __forceinline__ void slice_tail(U* buf, int off, const U* src, uint32_t g0, int len,
+                                           uint64_t n, int tid) {
+  constexpr uint64_t V = 16 / sizeof(U);
+  const uint64_t g = n / V * V + tid;  // at most V - 1 items
+  if (tid < (int)V && g >= g0 && g < (uint64_t)g0 + len) buf[off + (int)(g - g0)] = src[g];
+}
+
+// Fetches both slices into buf; all threads call it, the items are there
+// after it returns (block barrier inside).  `phase`: the barrier's parity.
+template <class U, int THREADS>
+__device__ __forceinline__ void tile_fetch(U* buf, const TileSlices& t, const U* l, const U* r,
+                                           uint64_t nl, uint64_t nr, bool aligned, uint64_t* bar,
+                                           uint32_t phase, const DevErr& err) {
+  const int tid = threadIdx.x;
+  if (aligned) {
+    if (tid == 0) {
+      const uint32_t ba = slice_bytes<U>(t.i0, t.la, nl), bb = slice_bytes<U>(t.j0, t.lb, nr);
+      fence_proxy_async_smem();
+      mbar_arrive_expect_tx(bar, ba + bb);
+      slice_load<U>(buf, t.a_off, l, t.i0, ba, bar);
+      slice_load<U>(buf, t.b_off, r, t.j0, bb, bar);
+    }
+    slice_tail<U>(buf, t.a_off, l, t.i0, t.la, nl, tid);
+    slice_tail<U>(buf, t.b_off, r, t.j0, t.lb, nr, tid);
+    if (!mbar_wait(bar, phase)) raise_device_error(err, MB_DEV_ERR_LOOKBACK);
+  } else {
+    for (int k = tid; k < t.la; k += THREADS) buf[t.a_off + k] = l[t.i0 + k];
+    for (int k = tid; k < t.lb; k += THREADS) buf[t.b_off + k] = r[t.j0 + k];
+  }
+  __syncthreads();
+}
+
+// The split of diagonal d of a tile in shared memory, by one warp: 33
+// sub-ranges per round, three rounds for any tile.
+template <class U, int ENC>
+__device__ __forceinline__ int warp_split(const U* a, int la, const U* b, int lb, int d, U flip) {
+  const int lane = (int)lane_id();
+  int lo = d > lb ? d - lb : 0, hi = d < la ? d : la;
+  while (lo < hi) {  // warp-uniform
+    const int step = (hi - lo + 32) / 33;
+    const int mid = lo + (lane + 1) * step - 1;
+    const bool before =
+        mid < hi && ord_of<U, ENC>(a[mid], flip) <= ord_of<U, ENC>(b[d - 1 - mid], flip);
+    const uint32_t m = __ballot_sync(kFull, before);
+    lo += __popc(m) * step;
+    if (m != kFull) hi = min(hi, lo + step - 1);
+  }
+  return lo;
+}
+
+// ---- merge: a tile per CTA, kMergeSeg outputs per warp, windows of 64 ----
+//
+// The window's 64 smallest items come out of the reversed comparison as a
+// bitonic sequence and are sorted by one in-register and five shuffle steps.
+// Equal words are equal items here, so which input a tied item came from
+// cannot be seen.  A window past the end of a slice reads the largest word;
+// should it be taken for an equal real item, the same values come out.
+// 8 warps x 4 KB: with 32 KB tiles six CTAs share an SM.
+constexpr int kMergeWarpBytes = 4096;
+
+template <class U>
+struct MergeCfg {
+  static constexpr int SEG = kMergeWarpBytes / (int)sizeof(U);
+  static constexpr int TILE = SEG * (kThreads / 32);
+  static constexpr int BUF = TILE + 4 * (16 / (int)sizeof(U));
+};
+
+template <class U, int ENC>
+__global__ void __launch_bounds__(kThreads)
+    merge_window_kernel(Src L, Src R, U* __restrict__ out, U flip, bool aligned,
+                        const uint32_t* __restrict__ splits, DevErr err) {
+  using C = MergeCfg<U>;
+  __shared__ __align__(16) U buf[C::BUF];
+  __shared__ __align__(8) uint64_t bar;
+  const uint64_t nl = src_len(L), nr = src_len(R), n = nl + nr;
+  const uint64_t d0 = (uint64_t)blockIdx.x * C::TILE;
+  if (d0 >= n) return;
+  const uint64_t d1 = min(d0 + (uint64_t)C::TILE, n);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    mbar_init(&bar, 1);
+    mbar_init_fence();
+  }
+  const TileSlices t = tile_slices<U>(d0, d1, splits[blockIdx.x], splits[blockIdx.x + 1]);
+  __syncthreads();
+  tile_fetch<U, kThreads>(buf, t, (const U*)L.data, (const U*)R.data, nl, nr, aligned, &bar, 0,
+                          err);
+  const U* sa = buf + t.a_off;
+  const U* sb = buf + t.b_off;
+  const int total = t.la + t.lb;
+  const int w0 = warp * C::SEG;
+  if (w0 >= total) return;
+  int a = warp_split<U, ENC>(sa, t.la, sb, t.lb, w0, flip);
+  int b = w0 - a;
+  const int w1 = min(w0 + C::SEG, total);
+  constexpr U kMax = ~(U)0;
+  U* o = out + d0;
+  for (int d = w0; d < w1; d += 64) {
+    const int ia = a + lane, ib = b + 31 - lane;
+    const U a0 = ia < t.la ? ord_of<U, ENC>(sa[ia], flip) : kMax;
+    const U a1 = ia + 32 < t.la ? ord_of<U, ENC>(sa[ia + 32], flip) : kMax;
+    const U b1 = ib < t.lb ? ord_of<U, ENC>(sb[ib], flip) : kMax;
+    const U b0 = ib + 32 < t.lb ? ord_of<U, ENC>(sb[ib + 32], flip) : kMax;
+    const int ca = __popc(__ballot_sync(kFull, a0 <= b0)) + __popc(__ballot_sync(kFull, a1 <= b1));
+    a += ca;
+    b += 64 - ca;
+    U x = min(a0, b0), y = min(a1, b1);
+    const U lo = min(x, y);
+    y = max(x, y);
+    x = lo;
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+      const U ox = __shfl_xor_sync(kFull, x, s), oy = __shfl_xor_sync(kFull, y, s);
+      const bool up = (lane & s) != 0;
+      x = up ? max(x, ox) : min(x, ox);
+      y = up ? max(y, oy) : min(y, oy);
+    }
+    if (d + lane < w1) __stcs(o + d + lane, ord_to_raw<U, ENC>(x, flip));
+    if (d + 32 + lane < w1) __stcs(o + d + 32 + lane, ord_to_raw<U, ENC>(y, flip));
+  }
+}
+
+// ---- intersection / difference: only the left items are wanted ----------
+//
+// The r-th copy (r from 0) of a value in the left input has a partner when
+// the right input's r-th copy exists: right[lower_bound(right, v) + r] == v.
+// Intersection keeps the items with a partner, difference the others.  A
+// window of 32 left and 32 right items gives the split of the next 32 merged
+// items; each left item taken in it finds its lower bound among the window's
+// right items by five shuffles, its r from the run heads of the window
+// (ballot) or the run start carried from the windows before, and its partner
+// with one read of the right slice (global memory past the slice's end).  At
+// the start of a warp's segment the run start is looked up in the 32 left
+// items before it, and by a search when they are all equal.  Kept items are
+// compacted over the warp's own left items, which no other warp reads, then
+// written behind the count of all earlier tiles (decoupled look-back).
+// CTAs take tiles from a ticket until none is left, so a capacity far above
+// the device length costs no launch of empty blocks.
+constexpr int kSetWarpBytes = 2048;  // 16 KB tiles
+
+template <class U>
+struct SetCfg {
+  static constexpr int SEG = kSetWarpBytes / (int)sizeof(U);
+  static constexpr int TILE = SEG * (kThreads / 32);
+  static constexpr int BUF = TILE + 4 * (16 / (int)sizeof(U));
+};
+
+// First index in [0, hi] of the run of `v` that reaches index hi (ordered
+// words of a sorted column), by one warp.
+template <class U, int ENC>
+__device__ uint32_t warp_run_start(const U* __restrict__ x, uint32_t hi, U v, U flip) {
+  const uint32_t lane = lane_id();
+  uint64_t lo = 0, top = hi;
+  while (lo < top) {
+    const uint64_t step = (top - lo + 32) / 33;
+    const uint64_t mid = lo + (uint64_t)(lane + 1) * step - 1;
+    const bool before = mid < top && ord_of<U, ENC>(x[mid], flip) < v;
+    const uint32_t m = __ballot_sync(kFull, before);
+    lo += (uint64_t)__popc(m) * step;
+    if (m != kFull) top = min(top, lo + step - 1);
+  }
+  return (uint32_t)lo;
+}
+
+template <class U, int ENC>
+__global__ void __launch_bounds__(kThreads, 6)
+    set_window_kernel(bool difference, Src L, Src R, U* __restrict__ out, U flip, bool aligned,
+                      uint32_t* count_dev, const uint32_t* __restrict__ splits, uint32_t* counter,
+                      TileState<uint32_t, true> st, DevErr err) {
+  using C = SetCfg<U>;
+  constexpr int W = kThreads / 32;
+  __shared__ __align__(16) U buf[C::BUF];
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ uint32_t s_tile, s_excl;
+  __shared__ int s_split[W + 1];
+  __shared__ uint32_t s_kept[W];
+  const uint64_t nl = src_len(L), nr = src_len(R), n = nl + nr;
+  const U* lg = (const U*)L.data;
+  const U* rg = (const U*)R.data;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr U kMax = ~(U)0;
+  if (tid == 0) {
+    mbar_init(&bar, 1);
+    mbar_init_fence();
+  }
+  for (uint32_t phase = 0;; phase ^= 1) {
+    if (tid == 0) s_tile = atomicAdd(counter, 1u);
+    __syncthreads();
+    const uint64_t tile = s_tile;
+    const uint64_t d0 = tile * (uint64_t)C::TILE;
+    if (d0 >= n) return;
+    const uint64_t d1 = min(d0 + (uint64_t)C::TILE, n);
+    const TileSlices t = tile_slices<U>(d0, d1, splits[tile], splits[tile + 1]);
+    tile_fetch<U, kThreads>(buf, t, lg, rg, nl, nr, aligned, &bar, phase, err);
+    U* sa = buf + t.a_off;
+    const U* sb = buf + t.b_off;
+    const int total = t.la + t.lb;
+    const int w0 = min(warp * C::SEG, total);
+    int a = warp_split<U, ENC>(sa, t.la, sb, t.lb, w0, flip);
+    if (lane == 0) s_split[warp] = a;
+    if (tid == 0) s_split[W] = t.la;
+    __syncthreads();
+    int b = w0 - a;
+    const int a0 = a, a1 = s_split[warp + 1];
+    int kept = 0;
+    if (a < a1) {
+      // run start of the segment's first left item
+      uint32_t run = t.i0 + (uint32_t)a;
+      U prev = ord_of<U, ENC>(sa[a], flip);
+      bool cont = false;  // the first item continues a run
+      {
+        const bool in = run > (uint32_t)lane;
+        const bool eq = in && ord_of<U, ENC>(lg[run - 1 - lane], flip) == prev;
+        const uint32_t ne = __ballot_sync(kFull, !eq);
+        if (ne) {
+          const uint32_t back = (uint32_t)__ffs(ne) - 1u;
+          cont = back > 0;
+          run -= back;
+        } else {
+          cont = true;
+          run = warp_run_start<U, ENC>(lg, run - 32, prev, flip);
+        }
+      }
+      while (a < a1) {
+        const bool va = a + lane < a1, vb = b + lane < t.lb;
+        const U raw = va ? sa[a + lane] : U(0);
+        const U ka = ord_of<U, ENC>(raw, flip);
+        const U kb = vb ? ord_of<U, ENC>(sb[b + lane], flip) : kMax;
+        const U rb = __shfl_xor_sync(kFull, kb, 31);
+        const bool rv = b + 31 - lane < t.lb;
+        const int ca = __popc(__ballot_sync(kFull, va && (!rv || ka <= rb)));
+        // right items of the window below this left item (at most 31)
+        int pos = 0;
+#pragma unroll
+        for (int s = 16; s >= 1; s >>= 1) {
+          const U p = __shfl_sync(kFull, kb, pos + s - 1);
+          if (p < ka) pos += s;
+        }
+        // run of this left item
+        const U up = __shfl_up_sync(kFull, ka, 1);
+        const bool head = lane == 0 ? !(cont && ka == prev) : ka != up;
+        const uint32_t heads = __ballot_sync(kFull, head) & (kFull >> (31 - lane));
+        const uint32_t me = t.i0 + (uint32_t)(a + lane);
+        const uint32_t start = heads ? t.i0 + (uint32_t)(a + 31 - __clz(heads)) : run;
+        // its partner on the right
+        bool keep = false;
+        if (lane < ca) {
+          const uint64_t p = (uint64_t)(b + pos) + (me - start);  // in the right slice
+          if (p < (uint64_t)t.lb)
+            keep = ord_of<U, ENC>(sb[p], flip) == ka;
+          else if (t.j0 + p < nr)
+            keep = ord_of<U, ENC>(rg[t.j0 + p], flip) == ka;
+          keep = keep != difference;
+        }
+        const uint32_t km = __ballot_sync(kFull, keep);
+        if (keep) sa[a0 + kept + __popc(km & ((1u << lane) - 1u))] = raw;
+        kept += __popc(km);
+        if (ca > 0) {
+          prev = __shfl_sync(kFull, ka, ca - 1);
+          run = __shfl_sync(kFull, start, ca - 1);
+          cont = true;
+        }
+        a += ca;
+        b += 32 - ca;
+      }
+    }
+    if (lane == 0) s_kept[warp] = (uint32_t)kept;
+    __syncthreads();
+    if (warp == 0) {
+      const uint32_t agg = __reduce_add_sync(kFull, lane < W ? s_kept[lane] : 0u);
+      const Op<uint32_t, MB_OP_ADD> add{MB_OP_ADD};
+      uint32_t excl = 0;
+      if (tile == 0) {
+        if (lane == 0) st.publish(0, kFlagIncl, agg);
+      } else {
+        if (lane == 0) st.publish(tile, kFlagAgg, agg);
+        excl = lookback_exclusive<uint32_t, Op<uint32_t, MB_OP_ADD>, false>(st, tile, add, err, 0u);
+        if (lane == 0) st.publish(tile, kFlagIncl, excl + agg);
+      }
+      if (lane == 0) {
+        s_excl = excl;
+        if (d1 == n && count_dev) *count_dev = excl + agg;
+      }
+    }
+    __syncthreads();
+    uint64_t base = s_excl;
+    for (int w = 0; w < warp; ++w) base += s_kept[w];
+    for (int k = lane; k < kept; k += 32) {
+      if (base + k < nl) out[base + k] = sa[a0 + k];
+      else raise_device_error(err, MB_DEV_ERR_BOUNDS);  // only after a failed look-back
+    }
+    __syncthreads();  // buf, s_tile and s_split are free again
+  }
+}
+
+// Whether the warp-window kernels take these inputs, and how they order them:
+// plain 4- and 8-byte columns.  `ties`: items that tie must also be equal
+// (merge writes whichever it meets), so floats only in the total order.
+template <class T>
+bool window_order(const mb_src& l, const mb_src& r, int less, bool ties, int& enc,
+                  typename UnsignedOf<T>::type& flip) {
+  using U = typename UnsignedOf<T>::type;
+  const int ct = DTypeOf<T>::value;
+  if (!src_plain(l, ct) || !src_plain(r, ct)) return false;
+  constexpr U sign = (U)1 << (sizeof(U) * 8 - 1);
+  flip = less == MB_GREATER ? ~(U)0 : (U)0;
+  if constexpr (std::is_floating_point<T>::value) {
+    if (ties && less != MB_TOTAL_LESS) return false;
+    enc = less == MB_TOTAL_LESS ? 2 : 1;
+  } else {
+    enc = 0;
+    if (std::is_signed<T>::value) flip ^= sign;
+  }
+  return true;
+}
+
+inline bool aligned16(const mb_src& l, const mb_src& r) {
+  return (uintptr_t)l.data % 16 == 0 && (uintptr_t)r.data % 16 == 0;
+}
+
+template <class U, int ENC>
+int window_splits(mb_executor* ex, const mb_src& l, const mb_src& r, uint32_t tile_items,
+                  uint64_t tiles, U flip, uint32_t* splits) {
+  const uint64_t threads = (tiles + 1) * kSplitLanes;
+  window_splits_kernel<U, ENC>
+      <<<(unsigned)((threads + kThreads - 1) / kThreads), kThreads, 0, ex->stream>>>(
+          to_src(l), to_src(r), tile_items, tiles, flip, splits);
+  MB_CUDA(cudaGetLastError());
+  return MB_OK;
+}
+
+template <class U, int ENC>
+int merge_window(mb_executor* ex, const mb_src& l, const mb_src& r, U flip, void* out) {
+  using C = MergeCfg<U>;
+  const uint64_t tiles = (l.len + r.len + C::TILE - 1) / C::TILE;
+  // [abort word, zeroed][splits]
+  Scratch scratch;
+  MB_TRY(scratch.alloc(ex, 256 + (tiles + 1) * sizeof(uint32_t)));
+  MB_CUDA(cudaMemsetAsync(scratch.ptr, 0, 4, ex->stream));
+  uint32_t* splits = scratch.as<uint32_t>() + 64;
+  MB_TRY((window_splits<U, ENC>(ex, l, r, C::TILE, tiles, flip, splits)));
+  merge_window_kernel<U, ENC><<<(unsigned)tiles, kThreads, 0, ex->stream>>>(
+      to_src(l), to_src(r), (U*)out, flip, aligned16(l, r), splits,
+      DevErr{ex->status_dev, scratch.as<uint32_t>()});
+  MB_CUDA(cudaGetLastError());
+  return MB_OK;
+}
+
+template <class U, int ENC>
+int set_window(mb_executor* ex, const mb_src& l, const mb_src& r, bool difference, U flip,
+               void* out, uint32_t* count_dev) {
+  using C = SetCfg<U>;
+  const uint64_t tiles = (l.len + r.len + C::TILE - 1) / C::TILE;
+  const size_t state_b = TileState<uint32_t, true>::bytes(tiles);
+  Scratch scratch;
+  MB_TRY(scratch.alloc(ex, 256 + state_b + (tiles + 1) * sizeof(uint32_t)));
+  char* base = scratch.as<char>();
+  MB_CUDA(cudaMemsetAsync(base, 0, 256 + state_b, ex->stream));
+  uint32_t* splits = (uint32_t*)(base + 256 + state_b);
+  MB_TRY((window_splits<U, ENC>(ex, l, r, C::TILE, tiles, flip, splits)));
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ex->device);
+  const uint64_t grid = std::min<uint64_t>(tiles, (uint64_t)sms * 6);  // 6 CTAs per SM reside
+  set_window_kernel<U, ENC><<<(unsigned)grid, kThreads, 0, ex->stream>>>(
+      difference, to_src(l), to_src(r), (U*)out, flip, aligned16(l, r), count_dev, splits,
+      (uint32_t*)base, TileState<uint32_t, true>::make(base + 256, tiles),
+      DevErr{ex->status_dev, (uint32_t*)base + 1});
+  MB_CUDA(cudaGetLastError());
+  return MB_OK;
+}
+
 template <class T, int LESS, bool PLAIN>
 int merge_launch(mb_executor* ex, const mb_src& l, const mb_src& r, void* out, int out_dtype,
                  const Payload& pay, uint32_t* count_dev) {
@@ -512,6 +1003,15 @@ int merge_less(mb_executor* ex, const mb_src& l, const mb_src& r, void* out, int
 template <class T>
 int merge_run(mb_executor* ex, const mb_src& l, const mb_src& r, int less, void* out,
               int out_dtype, const Payload& pay, uint32_t* count_dev) {
+  // Keys alone, element type kept: the warp-window kernel (floats under LESS
+  // and GREATER, where -0 and +0 tie, need to know the side of each item).
+  using U = typename UnsignedOf<T>::type;
+  constexpr int kBijection = std::is_floating_point<T>::value ? 2 : 0;
+  int enc = 0;
+  U flip = 0;
+  if (pay.ncols == 0 && !count_dev && out && out_dtype == DTypeOf<T>::value &&
+      window_order<T>(l, r, less, true, enc, flip))
+    return merge_window<U, kBijection>(ex, l, r, flip, out);
   switch (less) {
     case MB_GREATER: return merge_less<T, MB_GREATER>(ex, l, r, out, out_dtype, pay, count_dev);
     case MB_TOTAL_LESS:
@@ -554,6 +1054,17 @@ int set_launch(mb_executor* ex, const mb_src& l, const mb_src& r, int mode, cons
 template <class T>
 int set_run(mb_executor* ex, const mb_src& l, const mb_src& r, int less, int mode,
             const mb_col& out, uint32_t* count_dev) {
+  using U = typename UnsignedOf<T>::type;
+  int enc = 0;
+  U flip = 0;
+  if (mode != 0 && window_order<T>(l, r, less, false, enc, flip)) {
+    if constexpr (std::is_floating_point<T>::value) {
+      if (enc == 1) return set_window<U, 1>(ex, l, r, mode == 2, flip, out.data, count_dev);
+      return set_window<U, 2>(ex, l, r, mode == 2, flip, out.data, count_dev);
+    } else {
+      return set_window<U, 0>(ex, l, r, mode == 2, flip, out.data, count_dev);
+    }
+  }
   const int ct = DTypeOf<T>::value;
   const bool plain = src_plain(l, ct) && src_plain(r, ct);
 #define MB_SET_LESS(LESSID)                                                              \
