@@ -25,7 +25,7 @@
 #include "bulk.cuh"
 #include "common.cuh"
 #include "dispatch.cuh"
-#include "lookback.cuh"
+#include "lookback_group.cuh"
 
 namespace mb {
 
@@ -771,7 +771,7 @@ template <class U, int ENC>
 __global__ void __launch_bounds__(kThreads, 6)
     set_window_kernel(bool difference, Src L, Src R, U* __restrict__ out, U flip, bool aligned,
                       uint32_t* count_dev, const uint32_t* __restrict__ splits, uint32_t* counter,
-                      TileState<uint32_t, true> st, DevErr err) {
+                      TileState<uint32_t, true> st, GroupLines<uint32_t> lines, DevErr err) {
   using C = SetCfg<U>;
   constexpr int W = kThreads / 32;
   __shared__ __align__(16) U buf[C::BUF];
@@ -879,8 +879,7 @@ __global__ void __launch_bounds__(kThreads, 6)
         if (lane == 0) st.publish(0, kFlagIncl, agg);
       } else {
         if (lane == 0) st.publish(tile, kFlagAgg, agg);
-        excl = lookback_exclusive<uint32_t, Op<uint32_t, MB_OP_ADD>, false>(st, tile, add, err, 0u);
-        if (lane == 0) st.publish(tile, kFlagIncl, excl + agg);
+        excl = lookback_two_level<uint32_t>(st, lines, tile, add, err, 0u);
       }
       if (lane == 0) {
         s_excl = excl;
@@ -958,10 +957,11 @@ int set_window(mb_executor* ex, const mb_src& l, const mb_src& r, bool differenc
   const uint64_t tiles = (l.len + r.len + C::TILE - 1) / C::TILE;
   const size_t state_b = TileState<uint32_t, true>::bytes(tiles);
   Scratch scratch;
-  MB_TRY(scratch.alloc(ex, 256 + state_b + (tiles + 1) * sizeof(uint32_t)));
+  const size_t lines_b = GroupLines<uint32_t>::bytes(tiles);
+  MB_TRY(scratch.alloc(ex, 256 + state_b + lines_b + (tiles + 1) * sizeof(uint32_t)));
   char* base = scratch.as<char>();
-  MB_CUDA(cudaMemsetAsync(base, 0, 256 + state_b, ex->stream));
-  uint32_t* splits = (uint32_t*)(base + 256 + state_b);
+  MB_CUDA(cudaMemsetAsync(base, 0, 256 + state_b + lines_b, ex->stream));
+  uint32_t* splits = (uint32_t*)(base + 256 + state_b + lines_b);
   MB_TRY((window_splits<U, ENC>(ex, l, r, C::TILE, tiles, flip, splits)));
   int sms = 148;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ex->device);
@@ -969,7 +969,7 @@ int set_window(mb_executor* ex, const mb_src& l, const mb_src& r, bool differenc
   set_window_kernel<U, ENC><<<(unsigned)grid, kThreads, 0, ex->stream>>>(
       difference, to_src(l), to_src(r), (U*)out, flip, aligned16(l, r), count_dev, splits,
       (uint32_t*)base, TileState<uint32_t, true>::make(base + 256, tiles),
-      DevErr{ex->status_dev, (uint32_t*)base + 1});
+      GroupLines<uint32_t>{base + 256 + state_b}, DevErr{ex->status_dev, (uint32_t*)base + 1});
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }

@@ -32,7 +32,7 @@
 #include "bulk.cuh"
 #include "common.cuh"
 #include "dispatch.cuh"
-#include "lookback.cuh"
+#include "lookback_group.cuh"
 
 namespace mb {
 namespace {
@@ -77,6 +77,7 @@ struct ScanParams {
   T init;
   uint32_t* counter;
   DevErr err;
+  GroupLines<T> lines;
 };
 
 template <class T>
@@ -97,13 +98,28 @@ __device__ __forceinline__ void store_vec(T* p, uint64_t elem, const T (&src)[16
   __stcs(reinterpret_cast<uint4*>(p + elem), u);
 }
 
+// The look-back of a scan kernel: two-level (lookback_group.cuh), for which
+// tiles publish no inclusive prefix.  Float MIN / MAX and the run-time float
+// operators keep the left fold over tiles from the nearest inclusive prefix:
+// there the association decides what becomes of a NaN.
+template <class T, int OP>
+constexpr bool kTwoLevel = !std::is_floating_point<T>::value || OP == MB_OP_ADD;
+
+template <class T, int OP, bool PACKED>
+__device__ __forceinline__ T scan_lookback(const TileState<T, PACKED>& st,
+                                           const ScanParams<T>& p, uint64_t tile,
+                                           const Op<T, OP>& op, T fallback) {
+  if constexpr (kTwoLevel<T, OP>)
+    return lookback_two_level<T>(st, p.lines, tile, op, p.err, fallback);
+  else return lookback_exclusive<T, Op<T, OP>, true>(st, tile, op, p.err, fallback);
+}
+
 // Warp 0: folds the warp totals, publishes the tile, runs the look-back and
 // writes each warp's prefix (pre[w], has[w]).
 template <class T, int OP, bool PACKED>
 __device__ __forceinline__ void tile_prefixes(uint64_t tile, const ScanParams<T>& p,
                                               const TileState<T, PACKED>& st, const T* wtot,
                                               T* pre, bool* has) {
-  constexpr bool DET = std::is_floating_point<T>::value;
   const Op<T, OP> op{p.op};
   const int lane = threadIdx.x & 31;
   T agg = wtot[0];
@@ -114,10 +130,8 @@ __device__ __forceinline__ void tile_prefixes(uint64_t tile, const ScanParams<T>
     if (lane == 0) st.publish(0, kFlagIncl, agg);
   } else {
     if (lane == 0) st.publish(tile, kFlagAgg, agg);
-    // Floats: the fold-forward look-back (lookback.cuh); its per-tile
-    // inclusive prefixes keep the look-back short for these 32 KB tiles.
-    excl = lookback_exclusive<T, Op<T, OP>, DET>(st, tile, op, p.err, agg);
-    if (lane == 0) st.publish(tile, kFlagIncl, op(excl, agg));
+    excl = scan_lookback<T, OP, PACKED>(st, p, tile, op, agg);
+    if (!kTwoLevel<T, OP> && lane == 0) st.publish(tile, kFlagIncl, op(excl, agg));
   }
   if (lane == 0) {
     bool h = tile > 0;
@@ -281,7 +295,6 @@ template <class T, int OP, bool PACKED, class C>
 __global__ void __launch_bounds__(kThreads + 32)
     scan_smem_lb_kernel(const T* __restrict__ in, T* __restrict__ out, uint64_t n,
                         ScanParams<T> p, TileState<T, PACKED> st) {
-  constexpr bool DET = std::is_floating_point<T>::value;
   extern __shared__ __align__(128) unsigned char scan_smem[];
   T* buf = reinterpret_cast<T*>(scan_smem);
   __shared__ __align__(8) uint64_t bar;
@@ -311,7 +324,7 @@ __global__ void __launch_bounds__(kThreads + 32)
   if (warp == kWarps) {
     // the look-back warp
     T excl = T(0);
-    if (tile > 0) excl = lookback_exclusive<T, Op<T, OP>, DET>(st, tile, op, p.err, T(0));
+    if (tile > 0) excl = scan_lookback<T, OP, PACKED>(st, p, tile, op, T(0));
     if ((threadIdx.x & 31) == 0) s_excl = excl;
   } else {
     if (full) {
@@ -344,7 +357,7 @@ __global__ void __launch_bounds__(kThreads + 32)
       h = true;
       if (w > 0) agg = op(agg, s_wtot[w]);
     }
-    if (tile > 0) st.publish(tile, kFlagIncl, op(excl, agg));
+    if (!kTwoLevel<T, OP> && tile > 0) st.publish(tile, kFlagIncl, op(excl, agg));
   }
   named_sync(1, kThreads);
   smem_phase3<T, OP, C>(buf, tile, n, full, out, p, s_pre, s_has);
@@ -357,7 +370,6 @@ __device__ __forceinline__ void scan_tile(T (&x)[kLoads][16 / sizeof(T)], uint64
                                           const ScanParams<T>& p,
                                           const TileState<T, PACKED>& st, ScanShared<T>& sh) {
   constexpr int VEC = 16 / sizeof(T);
-  constexpr bool DET = std::is_floating_point<T>::value;
   const Op<T, OP> op{p.op};
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -395,9 +407,9 @@ __device__ __forceinline__ void scan_tile(T (&x)[kLoads][16 / sizeof(T)], uint64
       if (lane == 0) st.publish(0, kFlagIncl, agg);
     } else {
       if (lane == 0) st.publish(tile, kFlagAgg, agg);
-      T excl = lookback_exclusive<T, Op<T, OP>, DET>(st, tile, op, p.err, agg);
+      T excl = scan_lookback<T, OP, PACKED>(st, p, tile, op, agg);
       if (lane == 0) {
-        st.publish(tile, kFlagIncl, op(excl, agg));
+        if (!kTwoLevel<T, OP>) st.publish(tile, kFlagIncl, op(excl, agg));
         sh.excl = excl;
       }
     }
@@ -520,8 +532,9 @@ int scan_run(mb_executor* ex, const mb_src& in, int op, bool exclusive, const vo
   const uint64_t tiles = (cap + tile_items - 1) / tile_items;
   Scratch scratch;
   const size_t state_bytes = TileState<T, PACKED>::bytes(tiles);
-  MB_TRY(scratch.alloc(ex, 256 + state_bytes));
-  MB_CUDA(cudaMemsetAsync(scratch.ptr, 0, 256 + state_bytes, ex->stream));
+  const size_t need = 256 + state_bytes + GroupLines<T>::bytes(tiles);
+  MB_TRY(scratch.alloc(ex, need));
+  MB_CUDA(cudaMemsetAsync(scratch.ptr, 0, need, ex->stream));
   ScanParams<T> p{};
   p.op = op;
   p.exclusive = exclusive ? 1 : 0;
@@ -531,6 +544,7 @@ int scan_run(mb_executor* ex, const mb_src& in, int op, bool exclusive, const vo
   p.counter = scratch.as<uint32_t>();
   p.err = DevErr{ex->status_dev, scratch.as<uint32_t>() + 1};
   auto st = TileState<T, PACKED>::make(scratch.as<char>() + 256, tiles);
+  p.lines.base = scratch.as<char>() + 256 + state_bytes;
   const Src s = to_src(in);
   dim3 grid(grid_for(tiles)), block(kThreads);
   const size_t smem = shape == 2 ? BigCfg<T>::TILE_BYTES : SmemCfg<T>::TILE_BYTES;
@@ -660,7 +674,8 @@ int scan_noalloc_run(mb_executor* ex, const mb_src& in, int op, const mb_col& ou
   const bool smem_path = plain && in.len_dev == nullptr;
   const uint64_t tile_items = smem_path ? SmemCfg<T>::TILE : ScanCfg<T>::TILE;
   const uint64_t tiles = (cap + tile_items - 1) / tile_items;
-  const size_t need = 256 + TileState<T, PACKED>::bytes(tiles);
+  const size_t state_bytes = TileState<T, PACKED>::bytes(tiles);
+  const size_t need = 256 + state_bytes + GroupLines<T>::bytes(tiles);
   if (need > kNoAllocBytes)
     return set_error(MB_ERR_LENGTH_TOO_LARGE, "allocation-free scan: input too large", cap);
   void* scratch = nullptr;
@@ -676,6 +691,7 @@ int scan_noalloc_run(mb_executor* ex, const mb_src& in, int op, const mb_col& ou
   p.counter = (uint32_t*)scratch;
   p.err = DevErr{ex->status_dev, (uint32_t*)scratch + 1};
   auto st = TileState<T, PACKED>::make((char*)scratch + 256, tiles);
+  p.lines.base = (char*)scratch + 256 + state_bytes;
   const Src s = to_src(in);
   dim3 grid(grid_for(tiles)), block(kThreads);
   const size_t smem = SmemCfg<T>::TILE_BYTES;

@@ -20,7 +20,7 @@
 
 #include "bulk.cuh"
 #include "common.cuh"
-#include "lookback.cuh"
+#include "lookback_group.cuh"
 
 namespace mb {
 
@@ -49,6 +49,7 @@ struct SelParams {
   const uint32_t* boundary_dev;  // partition: number of kept rows
   uint32_t* counter;
   DevErr err;
+  GroupLines<uint32_t> lines;
 };
 
 __device__ __forceinline__ void st_raw(void* p, uint64_t i, int esize, uint64_t bits) {
@@ -115,9 +116,7 @@ __global__ void __launch_bounds__(kThreads) select_kernel(SelParams p, uint64_t 
       if (lane == 0) st.publish(0, kFlagIncl, agg);
     } else {
       if (lane == 0) st.publish(tile, kFlagAgg, agg);
-      excl = lookback_exclusive<uint32_t, Op<uint32_t, MB_OP_ADD>, false>(st, tile, add,
-                                                                           p.err, 0u);
-      if (lane == 0) st.publish(tile, kFlagIncl, excl + agg);
+      excl = lookback_two_level<uint32_t>(st, p.lines, tile, add, p.err, 0u);
     }
     if (lane == 0) {
       s_excl = excl;
@@ -197,7 +196,7 @@ __global__ void __launch_bounds__(kThreads + 32)
                        const uint32_t* __restrict__ stencil, uint32_t* __restrict__ out,
                        uint32_t* __restrict__ out1, uint64_t n, int fused_map, int in_dtype,
                        uint32_t invert, uint32_t* count_dev, uint32_t* counter, DevErr err,
-                       TileState<uint32_t, true> st) {
+                       TileState<uint32_t, true> st, GroupLines<uint32_t> lines) {
   constexpr int kCols = NCOL + (FUSED ? 0 : 1);
   constexpr int kTileBytes = kSmemTile * 4;
   extern __shared__ __align__(128) unsigned char sel_smem[];
@@ -234,7 +233,7 @@ __global__ void __launch_bounds__(kThreads + 32)
     uint32_t excl = 0;
     if (tile > 0) {
       const Op<uint32_t, MB_OP_ADD> add{MB_OP_ADD};
-      excl = lookback_exclusive<uint32_t, Op<uint32_t, MB_OP_ADD>, false>(st, tile, add, err, 0u);
+      excl = lookback_two_level<uint32_t>(st, lines, tile, add, err, 0u);
     }
     if (lane == 0) s_excl = excl;
   } else {
@@ -284,7 +283,6 @@ __global__ void __launch_bounds__(kThreads + 32)
   if (warp == kWarps) return;
   if (threadIdx.x == 0) {
     const uint32_t excl = s_excl, agg = s_agg;
-    if (tile > 0) st.publish(tile, kFlagIncl, excl + agg);
     if (tile_base + kSmemTile >= n && count_dev) *count_dev = excl + agg;
   }
   const uint32_t* wv = buf + warp * 32 * kSmemItems;
@@ -358,8 +356,11 @@ int select_entry(mb_executor* ex, const mb_src* in, int ncols, const mb_src* ste
     const bool fast = ncols == 1 && plain4;
     const uint64_t tiles = (n + kTile - 1) / kTile;
     Scratch scratch;
-    MB_TRY(scratch.alloc(ex, 256 + tiles * 8));
-    MB_CUDA(cudaMemsetAsync(scratch.ptr, 0, 256 + tiles * 8, ex->stream));
+    const size_t state_b = TileState<uint32_t, true>::bytes(tiles);
+    const size_t lines_b = GroupLines<uint32_t>::bytes(tiles);
+    MB_TRY(scratch.alloc(ex, 256 + state_b + lines_b));
+    MB_CUDA(cudaMemsetAsync(scratch.ptr, 0, 256 + state_b + lines_b, ex->stream));
+    p.lines.base = scratch.as<char>() + 256 + state_b;
     p.counter = scratch.as<uint32_t>();
     p.err = DevErr{ex->status_dev, scratch.as<uint32_t>() + 1};
     auto st = TileState<uint32_t, true>::make(scratch.as<char>() + 256, tiles);
@@ -379,7 +380,7 @@ int select_entry(mb_executor* ex, const mb_src* in, int ncols, const mb_src* ste
         kern<<<(unsigned)stiles, kThreads + 32, smem, ex->stream>>>(
             (const uint32_t*)in[0].data, in1, (const uint32_t*)stencil->data,
             (uint32_t*)out[0].data, out1, n, stencil->map, in[0].dtype,
-            mode == kRemove ? 1u : 0u, count_dev, p.counter, p.err, st);
+            mode == kRemove ? 1u : 0u, count_dev, p.counter, p.err, st, p.lines);
         MB_CUDA(cudaGetLastError());
         return MB_OK;
       };
