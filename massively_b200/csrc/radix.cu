@@ -36,7 +36,17 @@
 #include "lookback.cuh"
 
 namespace mb {
+
+uint64_t small_sort_max(int kdt);
+int small_sort(mb_executor* ex, int kdt, const void* ik, const void* iv, void* ok, void* ov,
+               size_t vsize, uint64_t n, const uint32_t* n_dev);
+
 namespace {
+
+bool wide_key(int kdt) {
+  return kdt == MB_U32 || kdt == MB_I32 || kdt == MB_F32 || kdt == MB_U64 || kdt == MB_I64 ||
+         kdt == MB_F64;
+}
 
 constexpr int kRadixBits = 8;
 constexpr int kBins = 1 << kRadixBits;
@@ -1060,6 +1070,10 @@ int bounded_wait_check(mb_executor* ex, int kind) {
 // the device by an earlier step; no host synchronisation).
 int radix_sort_plain(mb_executor* ex, int kdt, const void* ik, const void* iv, void* ok, void* ov,
                      size_t vsize, uint64_t n, const uint32_t* n_dev) {
+  // A column that fits one CTA (smallsort.cu), unless a shape was chosen.
+  if (ex->tune[MB_TUNE_RADIX] < 0 && wide_key(kdt) && (vsize == 0 || vsize == 4 || vsize == 8) &&
+      n <= small_sort_max(kdt))
+    return small_sort(ex, kdt, ik, iv, ok, ov, vsize, n, n_dev);
   switch (kdt) {
     case MB_U32: return sort_keys_vals<uint32_t, kEncUnsigned>(ex, ik, iv, ok, ov, vsize, n, n_dev);
     case MB_I32: return sort_keys_vals<uint32_t, kEncSigned>(ex, ik, iv, ok, ov, vsize, n, n_dev);
