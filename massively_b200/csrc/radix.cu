@@ -302,25 +302,35 @@ __global__ void __launch_bounds__(kBins)
                       void* out_k, void* tmp_k, const void* in_v, void* out_v, void* tmp_v) {
   if (n_dev && *n_dev < n) n = *n_dev;
   if (threadIdx.x == 0) plan->n = (uint32_t)n;
-  __shared__ uint32_t s_scan[kBins];
+  // All passes at once: their shuffle scans are independent, and two barriers
+  // serve every pass.
+  __shared__ uint32_t s_wsum[8][kBins / 32];
   __shared__ uint32_t s_trivial[8];
-  const int d = threadIdx.x;
-  for (int p = 0; p < passes; ++p) {
-    const uint32_t c = hist[p * kBins + d];
-    if (d == 0) s_trivial[p] = 0;
-    __syncthreads();
-    if ((uint64_t)c == n) s_trivial[p] = 1;
-    s_scan[d] = c;
-    __syncthreads();
-    for (int off = 1; off < kBins; off <<= 1) {
-      uint32_t v = d >= off ? s_scan[d - off] : 0;
-      __syncthreads();
-      s_scan[d] += v;
-      __syncthreads();
+  const int d = threadIdx.x, lane = d & 31, warp = d >> 5;
+  if (d < 8) s_trivial[d] = 0;
+  uint32_t c[8], incl[8];
+#pragma unroll
+  for (int p = 0; p < 8; ++p) incl[p] = c[p] = p < passes ? hist[p * kBins + d] : 0u;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1)
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+      const uint32_t o = __shfl_up_sync(kFull, incl[p], off);
+      if (lane >= off) incl[p] += o;
     }
-    hist[p * kBins + d] = s_scan[d] - c;  // exclusive offset
-    __syncthreads();
+#pragma unroll
+  for (int p = 0; p < 8; ++p)
+    if (lane == 31) s_wsum[p][warp] = incl[p];
+  __syncthreads();
+#pragma unroll
+  for (int p = 0; p < 8; ++p) {
+    if (p >= passes) continue;
+    if ((uint64_t)c[p] == n) s_trivial[p] = 1;
+    uint32_t before = incl[p] - c[p];
+    for (int w = 0; w < warp; ++w) before += s_wsum[p][w];
+    hist[p * kBins + d] = before;  // exclusive offset
   }
+  __syncthreads();
   if (d == 0) {
     int m = 0;
     for (int p = 0; p < passes; ++p) m += s_trivial[p] ? 0 : 1;
@@ -570,6 +580,18 @@ struct OnesweepTmaSmem {
   uint64_t bar;
 };
 
+// Rounds that find their peers by ballots although a mask table is there (one
+// table).  The mask table's three accesses per round are what fills the
+// shared-memory pipe, the ballots' logic what fills the ALU pipe, so a mix
+// loads both: 2^28 u32 pairs 6.38 ms with masks alone, 6.71 ms with ballots
+// alone, 6.10 / 6.07 / 6.31 ms with 4 / 8 / 12 of 16 rounds by ballots; 40 M
+// Zipf(1.1) pairs (few digits, many peers) 1.25 -> 1.08 ms.  64-bit keys,
+// 2^25: 1.86 / 1.77 / 1.78 / 1.89 ms with 0 / 4 / 8 / 12 rounds.
+template <class K>
+__device__ constexpr bool ballot_round(int k) {
+  return k % 4 < (sizeof(K) == 4 ? 2 : 1);
+}
+
 template <class K, int ENC, class V, int THREADS, int ITEMS, int NT, bool P64, bool FULL, class SW>
 __device__ __forceinline__ void onesweep_tile(OnesweepTmaSmem<K, V, THREADS, ITEMS, NT>& sm,
                                               const uint32_t tile, const uint32_t valid,
@@ -635,6 +657,20 @@ __device__ __forceinline__ void onesweep_tile(OnesweepTmaSmem<K, V, THREADS, ITE
       const uint32_t d =
           (FULL || li < valid) ? digit_of<K, ENC>(sm.keys[li], shift) : (uint32_t)kBins;
       rd[k] = d << 16;
+      if constexpr (NT == 1) {
+        if (ballot_round<K>(k)) {
+          constexpr int NB = FULL ? kRadixBits : kRadixBits + 1;
+          uint32_t eq = kFull;
+#pragma unroll
+          for (int b = 0; b < NB; ++b) {
+            const bool bit = (d >> b) & 1u;
+            const uint32_t bal = __ballot_sync(kFull, bit);
+            eq &= bit ? bal : ~bal;
+          }
+          peers[k] = eq;
+          continue;
+        }
+      }
       uint32_t* m = sm.mask[k % NT][warp];
       atomicOr(&m[d], me);
       __syncwarp();
