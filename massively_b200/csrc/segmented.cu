@@ -31,6 +31,10 @@
 namespace mb {
 
 int materialize(mb_executor* ex, const mb_src& in, void* dst);
+int seg_scan_carries(mb_executor* ex, int ct, const uint32_t* offsets, const uint32_t* tile_lb,
+                     uint64_t tiles, uint64_t tile_items, uint64_t cap, const uint32_t* n_dev,
+                     int op, int exclusive, const void* init, const void* part_tail, void* out,
+                     int out_dtype);
 
 namespace {
 
@@ -48,9 +52,9 @@ constexpr int kSegMinBlocks = 4;
 // seg_reduce_cross_kernel then folds in tile order.
 // kScanInclTiles / kScanExclTiles: the segmented scans over offsets without
 // the look-back -- every tile scans as if it started a segment and leaves
-// its tail fold; seg_tile_carry_kernel scans those folds over the tiles
-// (a segmented scan of one value per tile), and seg_scan_fix_kernel applies
-// each tile's carry to the items before its first segment start.
+// its tail fold; seg_scan_carries (segcarry.cu) scans those folds over the
+// tiles (a segmented scan of one value per tile) and applies each tile's carry
+// to the items before its first segment start.
 // kReduceKeysTiles: reduce_by_key the same way -- a first pass counts every
 // tile's run heads (seg_run_heads_kernel) and scans the counts into each
 // tile's first run index (seg_run_base_kernel); each tile then reduces the
@@ -432,7 +436,7 @@ __global__ void __launch_bounds__(kThreads, kSegMinBlocks)
           const V prev = k == 0 ? prev0 : y[j][k - 1].v;
           // (without the look-back, the items of a segment that came in from
           // an earlier tile keep their tile-local inclusive value here;
-          // seg_scan_fix_kernel turns it into the exclusive result)
+          // seg_scan_carries turns it into the exclusive result)
           o[j][k] = local && y[j][k].heads == 0 ? y[j][k].v
                                                 : (hd ? p.init : vop(p.init, prev));
         }
@@ -703,8 +707,7 @@ __global__ void __launch_bounds__(kCarryThreads)
 }
 
 // kReduceKeysTiles: the runs that cross tile edges.  One block scans
-// (has a head, tail fold) over the tiles -- the segmented scan of
-// seg_tile_carry_kernel -- so `run` is the fold of the run still open at the
+// (has a head, tail fold) over the tiles, a segmented scan, so `run` is the fold of the run still open at the
 // end of tile u - 1.  That run ends in the first later tile with a head
 // (after the fold of the items before that head, part_head) or at the end of
 // the data; it is written there unless it ended exactly at the end of a tile
@@ -826,124 +829,6 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// Whether tile t (items [t * tile_items, te)) holds a segment start: the
-// first start at or after its beginning lies before its end.
-__device__ __forceinline__ bool tile_has_start(const uint32_t* offsets, const uint32_t* tile_lb,
-                                               uint64_t t, uint64_t te) {
-  return (uint64_t)offsets[tile_lb[t]] < te;
-}
-
-
-// kScan*Tiles: carry[t] = the fold of the segment that enters tile t over
-// the items before t -- the value of an inclusive segmented scan, over the
-// tiles, of (tile holds a start, its tail fold) at tile t - 1.  One block;
-// each thread folds a contiguous run of tiles, a block scan (fixed shape)
-// joins the runs, and the threads walk their runs again, so the result is
-// the same from run to run.
-template <class V>
-__global__ void __launch_bounds__(kCarryThreads)
-    seg_tile_carry_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ tile_lb,
-                          uint64_t tiles, uint64_t tile_items, uint64_t cap,
-                          const uint32_t* __restrict__ n_dev, int op,
-                          const V* __restrict__ part_tail, V* __restrict__ carry) {
-  using T = SegVal<V>;
-  const SegOp<V, kOpDyn> sop{Op<V, kOpDyn>{op}};
-  const uint64_t n = n_dev ? min((uint64_t)*n_dev, cap) : cap;
-  const uint64_t live = (n + tile_items - 1) / tile_items < tiles ? (n + tile_items - 1) / tile_items
-                                                                  : tiles;
-  const uint64_t per = (live + kCarryThreads - 1) / kCarryThreads;
-  const uint64_t u0 = threadIdx.x * per, u1 = min(u0 + per, live);
-  auto item = [&](uint64_t u) -> T {
-    const uint64_t te = min((u + 1) * tile_items, n);
-    return T{tile_has_start(offsets, tile_lb, u, te) ? 1u : 0u, part_tail[u]};
-  };
-  T agg{0, V(0)};
-  bool has = false;
-  for (uint64_t u = u0; u < u1; ++u) {
-    const T x = item(u);
-    agg = has ? sop(agg, x) : x;
-    has = true;
-  }
-  __shared__ T s_v[kCarryThreads];
-  __shared__ int s_h[kCarryThreads];
-  s_v[threadIdx.x] = agg;
-  s_h[threadIdx.x] = has;
-  __syncthreads();
-  for (int d = 1; d < kCarryThreads; d <<= 1) {  // inclusive, in thread order
-    T x{};
-    int hx = 0;
-    if (threadIdx.x >= d && s_h[threadIdx.x - d]) {
-      x = s_h[threadIdx.x] ? sop(s_v[threadIdx.x - d], s_v[threadIdx.x]) : s_v[threadIdx.x - d];
-      hx = 1;
-    }
-    __syncthreads();
-    if (hx) {
-      s_v[threadIdx.x] = x;
-      s_h[threadIdx.x] = 1;
-    }
-    __syncthreads();
-  }
-  T run{0, V(0)};
-  bool rh = threadIdx.x > 0 && s_h[threadIdx.x - 1];
-  if (rh) run = s_v[threadIdx.x - 1];
-  for (uint64_t u = u0; u < u1; ++u) {
-    if (rh) carry[u] = run.v;
-    const T x = item(u);
-    run = rh ? sop(run, x) : x;
-    rh = true;
-  }
-}
-
-// kScan*Tiles: the items of tile t before its first segment start belong to
-// a segment that began in an earlier tile; the tile kernel left their
-// tile-local inclusive values in `out`.  Inclusive: carry op local;
-// exclusive: init op (carry op local of the item before), init op carry for
-// the tile's first item.  All loads come before the barrier, all stores
-// after it.
-template <class V>
-__global__ void __launch_bounds__(kThreads)
-    seg_scan_fix_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ tile_lb,
-                        uint64_t tile_items, uint64_t cap, const uint32_t* __restrict__ n_dev,
-                        int op, int exclusive, V init, const V* __restrict__ carry, void* out,
-                        int out_dtype) {
-  constexpr int MAXR = (int)(SegCfg<V>::TILE / kThreads);
-  const uint64_t t = blockIdx.x + 1;  // tile 0 starts with a segment
-  const uint64_t n = n_dev ? min((uint64_t)*n_dev, cap) : cap;
-  const uint64_t tb = t * tile_items;
-  if (tb >= n) return;
-  const uint64_t te = min(tb + tile_items, n);
-  const uint64_t first = min((uint64_t)offsets[tile_lb[t]], te);
-  if (first == tb) return;
-  const uint64_t len = first - tb;
-  const V c = carry[t];
-  Src o{};
-  o.kind = MB_SRC_COLUMN;
-  o.dtype = out_dtype;
-  o.vtype = DTypeOf<V>::value;
-  o.map = MB_UN_IDENTITY;
-  o.data = out;
-  o.len = cap;
-  V x[MAXR], xp[MAXR];
-#pragma unroll
-  for (int r = 0; r < MAXR; ++r) {
-    const uint64_t i = (uint64_t)r * kThreads + threadIdx.x;
-    if (i < len) {
-      x[r] = src_load<V>(o, tb + i);
-      if (exclusive && i > 0) xp[r] = src_load<V>(o, tb + i - 1);
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int r = 0; r < MAXR; ++r) {
-    const uint64_t i = (uint64_t)r * kThreads + threadIdx.x;
-    if (i >= len) continue;
-    V v;
-    if (!exclusive) v = op_apply_rt<V>(op, c, x[r]);
-    else v = op_apply_rt<V>(op, init, i == 0 ? c : op_apply_rt<V>(op, c, xp[r]));
-    st_cast<V>(out_dtype, out, tb + i, v);
-  }
-}
-
 // kReduceKeysTiles: run bases shared by the value columns of one
 // reduce_by_key call (`ptr` holds tiles + 1 words for the smallest tile;
 // `tile` is the tile size they were computed for, 0 before the first).
@@ -967,8 +852,7 @@ int seg_run(mb_executor* ex, const mb_src& in, SegParams<V> p, const void* init_
   const size_t state_b =
       pk ? TileState<T, true>::bytes(tiles) : TileState<T, false>::bytes(tiles);
   const size_t lb_b = p.offsets ? ((tiles + 1) * 4 + 255) / 256 * 256 : 0;
-  // kReduceTiles: part_head, part_tail, tail_seg; kScan*Tiles: part_tail and
-  // the carries (in the part_head slot).
+  // kReduceTiles: part_head, part_tail, tail_seg; kScan*Tiles: part_tail.
   const bool scan_tiles = p.mode == kScanInclTiles || p.mode == kScanExclTiles;
   const bool keys_tiles = p.mode == kReduceKeysTiles;
   const bool tiles_mode = p.mode == kReduceTiles || scan_tiles || keys_tiles;
@@ -1058,15 +942,9 @@ int seg_run(mb_executor* ex, const mb_src& in, SegParams<V> p, const void* init_
 #undef MB_SEG_LAUNCH
   MB_CUDA(cudaGetLastError());
   if (scan_tiles) {
-    seg_tile_carry_kernel<V><<<1, kCarryThreads, 0, ex->stream>>>(
-        p.offsets, p.tile_lb, tiles, C::TILE, cap, in.len_dev, p.op, p.part_tail, p.part_head);
-    MB_CUDA(cudaGetLastError());
-    if (tiles > 1) {
-      seg_scan_fix_kernel<V><<<(unsigned)(tiles - 1), kThreads, 0, ex->stream>>>(
-          p.offsets, p.tile_lb, C::TILE, cap, in.len_dev, p.op,
-          p.mode == kScanExclTiles ? 1 : 0, p.init, p.part_head, p.out, p.out_dtype);
-      MB_CUDA(cudaGetLastError());
-    }
+    MB_TRY(seg_scan_carries(ex, DTypeOf<V>::value, p.offsets, p.tile_lb, tiles, C::TILE, cap,
+                            in.len_dev, p.op, p.mode == kScanExclTiles ? 1 : 0, &p.init,
+                            p.part_tail, p.out, p.out_dtype));
   } else if (keys_tiles) {
     seg_rbk_walk_kernel<V><<<1, kCarryThreads, 0, ex->stream>>>(
         tiles, C::TILE, cap, in.len_dev, p.op, p.init, p.part_head, p.part_tail, p.first_pos,
