@@ -53,6 +53,7 @@ constexpr int kSsItems = 16;
 constexpr int kSsTile = kSsThreads * kSsItems;  // 4096 items
 constexpr int kSsRange = kSsTile / 2;           // 2048 start positions per range
 constexpr int kSsBins = 256;
+constexpr int kSsWordBits = 24;                 // of (segment, value) that a pack sorts by passes
 constexpr int kSsNT = 3;                        // lane-mask tables used in turn
 constexpr uint32_t kSsLongLimit = 1u << 17;     // longest segment one CTA sorts
 constexpr uint32_t kSsLongCtas = 2 * 148;
@@ -131,6 +132,8 @@ __device__ __forceinline__ uint32_t ss_block_excl(SsSmem<PAY>& sm, uint32_t v) {
 // before their reuse.  The lowest peer adds the group's size to the warp's
 // digit counter and its old value comes back through a shuffle before the
 // next round's atomics: the ranks are stable.
+// (Peers by ballots in every other round, which pays in the onesweep kernel,
+// cost 10% here.)
 template <bool PAY>
 __device__ __forceinline__ void ss_pass(SsSmem<PAY>& sm, uint32_t valid, int shift) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -323,52 +326,51 @@ __device__ __forceinline__ void ss_pack(SsSmem<PAY>& sm, const Src& in, const ui
     if (tid < kSsTile / 32) sm.hpre[tid] = ex;
   }
   __syncthreads();
-  uint32_t or_lo = 0, and_lo = ~0u, or_hi = 0, and_hi = ~0u;
+  // Which value bits differ between some two items.
+  uint32_t or_lo = 0, and_lo = ~0u;
 #pragma unroll
   for (int k = 0; k < kSsItems; ++k) {
-    const uint32_t p = (uint32_t)k * kSsThreads + tid;
-    if (p < len) {
-      const uint32_t w = p >> 5;
-      const uint32_t seg =
-          sm.hpre[w] + (uint32_t)__popc(sm.heads[w] & (0xFFFFFFFFu >> (31 - (p & 31)))) - 1u;
+    if ((uint32_t)k * kSsThreads + tid < len) {
       const uint32_t u = ss_encode<ENC>(raw[k], desc, ieee);
-      sm.keys[p] = ((uint64_t)seg << 32) | u;
-      if constexpr (PAY) sm.pay[p] = raw[k];
       or_lo |= u;
       and_lo &= u;
-      or_hi |= seg;
-      and_hi &= seg;
     }
   }
   or_lo = __reduce_or_sync(kFull, or_lo);
   and_lo = __reduce_and_sync(kFull, and_lo);
-  or_hi = __reduce_or_sync(kFull, or_hi);
-  and_hi = __reduce_and_sync(kFull, and_hi);
   if (lane == 0) {
     sm.red[warp][0] = or_lo;
     sm.red[warp][1] = and_lo;
-    sm.red[warp][2] = or_hi;
-    sm.red[warp][3] = and_hi;
   }
   __syncthreads();
-  uint32_t var_lo = 0, var_hi = 0;
+  uint32_t var_lo, same;
   {
-    uint32_t a = 0, b = ~0u, c = 0, e = ~0u;
+    uint32_t a = 0, b = ~0u;
 #pragma unroll
     for (int w = 0; w < kSsWarps; ++w) {
       a |= sm.red[w][0];
       b &= sm.red[w][1];
-      c |= sm.red[w][2];
-      e &= sm.red[w][3];
     }
-    var_lo = a ^ b;  // bits that differ between some two items
-    var_hi = c ^ e;
+    var_lo = a ^ b;
+    same = b;  // the value bits outside var_lo
   }
-  // The lowest of four varying value digits is left out of the passes
-  // (`low`): a pack's keys rarely agree on segment and the value's top three
-  // digits, and ss_fix_runs orders the few that do.  (Leaving out two digits
-  // saved a pass but made runs common enough that their fix-up cost more.)
-  uint32_t low = 0;
+  const uint32_t nseg =
+      sm.hpre[kSsTile / 32 - 1] + (uint32_t)__popc(sm.heads[kSsTile / 32 - 1]);
+  const int vb = 32 - __clz(var_lo), sb = nseg > 1 ? 32 - __clz(nseg - 1) : 0;
+
+  // The keys of the passes: segment within the pack above the value, of which
+  // only the bits up to the highest varying one count, so that the two lie
+  // together; and of that word only the top 24 bits are sorted, in three
+  // passes, where sorting the varying digits of segment and value one by one
+  // would take more.  ss_fix_runs then orders the runs that agree there: a
+  // segment of a few hundred items rarely has any.  (2^26 u32 in 2^20
+  // segments: 1.59 -> 1.40 ms; with 16 bits 1.36 ms, but then floats, whose top bits are
+  // exponents, leave long runs.)  Otherwise the lowest of four varying value
+  // digits is left out in the same way: a pack's keys rarely agree on segment
+  // and the value's top three digits.  (Leaving out two digits saved a pass
+  // but made runs common enough that their fix-up cost more.)
+  uint32_t low = 0;  // the value bits left out
+  int digits = (sb + 7) / 8;
   {
     int m = 0, c = 0;
 #pragma unroll
@@ -377,31 +379,55 @@ __device__ __forceinline__ void ss_pack(SsSmem<PAY>& sm, const Src& in, const ui
     for (int j = 0; j < 4; ++j)
       if (((var_lo >> (8 * j)) & 0xFFu) && ++c == m - 3)
         low = j == 3 ? ~0u : ((1u << (8 * j + 8)) - 1u);
+    digits += m > 3 ? 3 : m;
   }
-  auto passes = [&](uint32_t vlo) {
-    for (int shift = 0; shift < 64; shift += 8) {
-      const uint32_t v = shift < 32 ? (vlo >> shift) : (var_hi >> (shift - 32));
-      if (v & 0xFFu) ss_pass(sm, len, shift);
-    }
+  static_assert(kSsTile <= 1 << 12, "a pack's segment numbers leave 12 bits of the word");
+  const int drop = max(0, sb + vb - kSsWordBits);
+  bool packed = (sb + vb - drop + 7) / 8 < digits;
+  if (packed) low = drop ? (1u << drop) - 1u : 0u;
+  const int up = packed ? vb : 32;
+  uint32_t vmask = up == 32 ? ~0u : (1u << up) - 1u;  // the value bits held in the key
+  auto segment_of = [&](uint32_t p) -> uint32_t {
+    const uint32_t w = p >> 5;
+    return sm.hpre[w] + (uint32_t)__popc(sm.heads[w] & (0xFFFFFFFFu >> (31 - (p & 31)))) - 1u;
   };
-  passes(var_lo & ~low);
-  if (low && !ss_fix_runs(sm, len, low)) {
+#pragma unroll
+  for (int k = 0; k < kSsItems; ++k) {
+    const uint32_t p = (uint32_t)k * kSsThreads + tid;
+    if (p < len) {
+      sm.keys[p] = ((uint64_t)segment_of(p) << up) | (ss_encode<ENC>(raw[k], desc, ieee) & vmask);
+      if constexpr (PAY) sm.pay[p] = raw[k];
+    }
+  }
+  __syncthreads();
+  while (true) {
+    for (int pass = 0; pass < 8; ++pass) {
+      int shift = 8 * pass;
+      if (packed) {
+        shift += drop;
+        if (shift >= sb + vb) break;
+      } else if (shift < 32 ? !((var_lo & ~low) >> shift & 0xFFu) : shift - 32 >= sb) {
+        continue;
+      }
+      ss_pass(sm, len, shift);
+    }
+    if (!low || ss_fix_runs(sm, len, low)) break;
     // A long run out of order: build the keys again and take every digit.
     for (uint32_t p = tid; p < len; p += kSsThreads) {
       const uint32_t r = ss_load<PLAIN>(in, (uint64_t)start + p);
-      const uint32_t w = p >> 5;
-      const uint32_t seg =
-          sm.hpre[w] + (uint32_t)__popc(sm.heads[w] & (0xFFFFFFFFu >> (31 - (p & 31)))) - 1u;
-      sm.keys[p] = ((uint64_t)seg << 32) | ss_encode<ENC>(r, desc, ieee);
+      sm.keys[p] = ((uint64_t)segment_of(p) << 32) | ss_encode<ENC>(r, desc, ieee);
       if constexpr (PAY) sm.pay[p] = r;
     }
     __syncthreads();
-    passes(var_lo);
+    packed = false;
+    low = 0;
+    vmask = ~0u;
   }
+  same &= ~vmask;
   for (uint32_t p = tid; p < len; p += kSsThreads) {
     uint32_t v;
     if constexpr (PAY) v = sm.pay[p];
-    else v = ss_decode<ENC>((uint32_t)sm.keys[p], desc);
+    else v = ss_decode<ENC>(((uint32_t)sm.keys[p] & vmask) | same, desc);
     out[(uint64_t)start + p] = v;
   }
   __syncthreads();  // shared memory is reused by the next pack
