@@ -1,24 +1,24 @@
 // merge.cu -- merge-path merge / merge_by_key and the multiset set
 // operations.
 //
-// Merge (massively/src/core/merge.rs:24-1230: a merge-path control kernel
-// of 64 threads x 4 items writing a permutation, then a separate apply pass
-// for the payload) becomes two: a small kernel finds the merge-path split of
-// every tile boundary (all binary searches at once), then every block reads
-// its two splits, stages its slice of both inputs in shared memory, each
-// thread finds its own split there and merges kItems outputs serially (an
-// odd count, so the threads' strided shared-memory accesses fall in distinct
-// banks), and the block writes keys and payload columns with coalesced
-// stores.  Ties take the left element first (vector.rs:493-513 of massively's
-// oracle: the right element is taken only when strictly less).
+// Merge (massively/src/core/merge.rs:24-1230: a merge-path control kernel of
+// 64 threads x 4 items writing a permutation, then a separate apply pass for
+// the payload) becomes two kernels: the merge-path splits of all tile
+// boundaries, then the tiles.  Plain keys alone take the warp-window kernel.
+// With payloads, lazy inputs, and floats under LESS / GREATER, each thread
+// finds its own split in shared memory and merges kItems outputs serially (an
+// odd count, so the threads' strided accesses fall in distinct banks).  Ties
+// take the left element first (vector.rs:493-513 of massively's oracle: the
+// right element is taken only when strictly less).
 //
 // Set operations (massively/src/core/set.rs:14-401) keep massively's
 // occurrence-rank rule: the k-th copy of a value in one input is kept by
 // intersection when the other input holds more than k copies, by difference
 // when it holds at most k; union is the merge of the left input with the
-// right input's extra copies.  Ranks and counts come from binary searches;
-// the kept elements are compacted by the single-pass selection kernel and the
-// result count stays on the device.
+// right input's extra copies.  Intersection and difference of plain columns
+// look each left item's partner up on the right (warp-window kernel); union
+// and the other inputs take one pass over the merged runs.  Kept items are
+// compacted behind a look-back and the result count stays on the device.
 
 #include <algorithm>
 
@@ -497,7 +497,9 @@ __global__ void __launch_bounds__(kThreads, 4)
 // window A and of window B reversed, compared lane by lane, give the split of
 // the next 32 x R outputs with one ballot per register (the merge-path
 // predicate is monotone along the diagonal), so there is no search per
-// thread and every shared-memory access is to consecutive words.
+// thread and every shared-memory access is to consecutive words.  Merge of
+// 100000007 and 150000001 u32: 788 -> 478 us (4.2 TB/s); set_intersection of
+// 33554393 and 30000001: 825 -> 420 us with its count read back.
 
 // Order- and equivalence-preserving map to unsigned words.  ENC: 0 integers
 // (raw ^ flip), 1 floats under LESS / GREATER, 2 floats in the total order;
@@ -525,37 +527,41 @@ __device__ __forceinline__ U ord_to_raw(U u, U flip) {
   return u;
 }
 
-// The merge-path split of every tile boundary by groups of eight lanes: nine
-// sub-ranges per round, so a 27-step binary search becomes nine rounds of
-// independent loads (the searches' latency, not their traffic, is what the
-// tile kernel waits for).  Boundaries past the logical end are not computed.
-constexpr int kSplitLanes = 8;
+// The merge-path split of every tile boundary by groups of G lanes, G + 1
+// sub-ranges per round.  Lists that stay in L2 take eight lanes: a 27-step
+// binary search becomes nine rounds of independent loads, and the searches'
+// latency is what the tile kernel waits for.  Longer lists take two (17
+// rounds): the probes are random DRAM reads, and wide rounds make more of them
+// (100000007 + 150000001 u32 merged in 523 / 510 / 496 us with 8 / 4 / 2 lanes,
+// 7000000 + 9000000 in 49 / 54 / 54 us).  Boundaries past the logical end are
+// not computed.
+constexpr uint64_t kSplitWideItems = 1ull << 26;
 
-template <class U, int ENC>
+template <class U, int ENC, int G>
 __global__ void __launch_bounds__(kThreads)
     window_splits_kernel(Src L, Src R, uint32_t tile_items, uint64_t tiles, U flip,
                          uint32_t* __restrict__ splits) {
   const uint64_t nl = src_len(L), nr = src_len(R), n = nl + nr;
   const U* l = (const U*)L.data;
   const U* r = (const U*)R.data;
-  const int lane = threadIdx.x & 31, sub = lane & (kSplitLanes - 1);
-  const int shift = lane & ~(kSplitLanes - 1);
-  const uint64_t b =
-      (blockIdx.x * (uint64_t)kThreads + threadIdx.x) / kSplitLanes;
+  const int lane = threadIdx.x & 31, sub = lane & (G - 1);
+  const int shift = lane & ~(G - 1);
+  constexpr uint32_t kAll = (1u << G) - 1u;
+  const uint64_t b = (blockIdx.x * (uint64_t)kThreads + threadIdx.x) / G;
   // (a boundary of the last, partial tile is still wanted: b * tile < n + tile)
   const bool on = b <= tiles && b * tile_items < n + tile_items;
   const uint64_t d = on ? min(b * tile_items, n) : 0;
   uint64_t lo = d > nr ? d - nr : 0, hi = d < nl ? d : nl;
   while (__any_sync(kFull, lo < hi)) {
-    const uint64_t step = (hi - lo + kSplitLanes) / (kSplitLanes + 1);
+    const uint64_t step = (hi - lo + G) / (G + 1);
     const uint64_t mid = lo + (uint64_t)(sub + 1) * step - 1;
     bool before = false;  // the split lies after mid
     if (lo < hi && mid < hi)
       before = ord_of<U, ENC>(l[mid], flip) <= ord_of<U, ENC>(r[d - 1 - mid], flip);
-    const uint32_t m = (__ballot_sync(kFull, before) >> shift) & ((1u << kSplitLanes) - 1u);
+    const uint32_t m = (__ballot_sync(kFull, before) >> shift) & kAll;
     if (lo < hi) {
       lo += (uint64_t)__popc(m) * step;
-      if (m != (1u << kSplitLanes) - 1u) hi = min(hi, lo + step - 1);
+      if (m != kAll) hi = min(hi, lo + step - 1);
     }
   }
   if (on && sub == 0) splits[b] = (uint32_t)lo;
@@ -660,8 +666,9 @@ __device__ __forceinline__ int warp_split(const U* a, int la, const U* b, int lb
 // Equal words are equal items here, so which input a tied item came from
 // cannot be seen.  A window past the end of a slice reads the largest word;
 // should it be taken for an equal real item, the same values come out.
-// 8 warps x 4 KB: with 32 KB tiles six CTAs share an SM.
-constexpr int kMergeWarpBytes = 4096;
+// 8 warps x 5.5 KB, five CTAs per SM: a tile pays its loads and the warps'
+// splits once (16 / 28 / 32 / 44 KB tiles: 603 / 513 / 496 / 478 us).
+constexpr int kMergeWarpBytes = 5632;
 
 template <class U>
 struct MergeCfg {
@@ -741,7 +748,9 @@ __global__ void __launch_bounds__(kThreads)
 // written behind the count of all earlier tiles (decoupled look-back).
 // CTAs take tiles from a ticket until none is left, so a capacity far above
 // the device length costs no launch of empty blocks.
-constexpr int kSetWarpBytes = 2048;  // 16 KB tiles
+// 32 KB tiles, six CTAs per SM (16 / 24 / 32 / 44 KB: 422 / 381 / 371 / 374 us;
+// 323 us without the look-back).
+constexpr int kSetWarpBytes = 4096;
 
 template <class U>
 struct SetCfg {
@@ -925,10 +934,11 @@ inline bool aligned16(const mb_src& l, const mb_src& r) {
 template <class U, int ENC>
 int window_splits(mb_executor* ex, const mb_src& l, const mb_src& r, uint32_t tile_items,
                   uint64_t tiles, U flip, uint32_t* splits) {
-  const uint64_t threads = (tiles + 1) * kSplitLanes;
-  window_splits_kernel<U, ENC>
-      <<<(unsigned)((threads + kThreads - 1) / kThreads), kThreads, 0, ex->stream>>>(
-          to_src(l), to_src(r), tile_items, tiles, flip, splits);
+  const bool wide = l.len + r.len >= kSplitWideItems;
+  const uint64_t threads = (tiles + 1) * (wide ? 2 : 8);
+  auto kern = wide ? window_splits_kernel<U, ENC, 2> : window_splits_kernel<U, ENC, 8>;
+  kern<<<(unsigned)((threads + kThreads - 1) / kThreads), kThreads, 0, ex->stream>>>(
+      to_src(l), to_src(r), tile_items, tiles, flip, splits);
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }
@@ -937,15 +947,13 @@ template <class U, int ENC>
 int merge_window(mb_executor* ex, const mb_src& l, const mb_src& r, U flip, void* out) {
   using C = MergeCfg<U>;
   const uint64_t tiles = (l.len + r.len + C::TILE - 1) / C::TILE;
-  // [abort word, zeroed][splits]
   Scratch scratch;
-  MB_TRY(scratch.alloc(ex, 256 + (tiles + 1) * sizeof(uint32_t)));
-  MB_CUDA(cudaMemsetAsync(scratch.ptr, 0, 4, ex->stream));
-  uint32_t* splits = scratch.as<uint32_t>() + 64;
+  MB_TRY(scratch.alloc(ex, (tiles + 1) * sizeof(uint32_t)));
+  uint32_t* splits = scratch.as<uint32_t>();
   MB_TRY((window_splits<U, ENC>(ex, l, r, C::TILE, tiles, flip, splits)));
   merge_window_kernel<U, ENC><<<(unsigned)tiles, kThreads, 0, ex->stream>>>(
       to_src(l), to_src(r), (U*)out, flip, aligned16(l, r), splits,
-      DevErr{ex->status_dev, scratch.as<uint32_t>()});
+      DevErr{ex->status_dev, nullptr});
   MB_CUDA(cudaGetLastError());
   return MB_OK;
 }

@@ -15,9 +15,9 @@
 //      scan of the vector, warp shuffle scan of the vector totals, carry from
 //      the previous row; the warp-local inclusive values go back to shared
 //      memory;
-//   2. warp 0 folds the eight warp totals in order, publishes the tile
-//      aggregate and runs the look-back (lookback.cuh), giving every warp its
-//      prefix;
+//   2. the eight warp totals are folded in order and the tile aggregate is
+//      published; a ninth warp runs the look-back (lookback_group.cuh), giving
+//      every warp its prefix;
 //   3. every value is combined with its warp prefix on the way out to global
 //      memory (16-byte streaming stores).
 // Lazy views and device-length inputs use a register-tiled kernel with the
@@ -59,15 +59,21 @@ struct TileCfg {
   static constexpr int TILE_BYTES = TILE * (int)sizeof(T);
 };
 
-// One-tile-per-CTA kernel.  Floats take 64 KB tiles: their deterministic
-// look-back folds one aggregate per tile in sequence, so fewer, larger tiles
-// shorten that chain.
+// One-tile-per-CTA kernel: 32 KB tiles, six per SM (2^28 f32 0.466 ms, with 64
+// KB tiles 0.477 ms).
 template <class T>
-struct SmemCfg : TileCfg<T, std::is_floating_point<T>::value ? 2 * kRows : kRows> {};
+struct SmemCfg : TileCfg<T, kRows> {};
 
-// Alternative shape for the autotuner: 64 KB tiles for every type.
+// 64 KB tiles: a shape for the autotuner, and what the float operators with a
+// left-fold look-back take (one step per tile in sequence, so fewer tiles
+// shorten the chain).
 template <class T>
 struct BigCfg : TileCfg<T, 2 * kRows> {};
+
+template <class T>
+bool left_fold(int op) {
+  return std::is_floating_point<T>::value && op != MB_OP_ADD;
+}
 
 template <class T>
 struct ScanParams {
@@ -524,7 +530,8 @@ int scan_run(mb_executor* ex, const mb_src& in, int op, bool exclusive, const vo
   const bool plain = src_plain(in, DTypeOf<T>::value) && out.dtype == DTypeOf<T>::value &&
                      ((uintptr_t)in.data % 16 == 0) && ((uintptr_t)out.data % 16 == 0);
   const bool smem_path = plain && in.len_dev == nullptr;
-  const int shape = smem_path ? std::max(0, ex->tune[MB_TUNE_SCAN]) : 0;
+  int shape = smem_path ? std::max(0, ex->tune[MB_TUNE_SCAN]) : 0;
+  if (smem_path && shape == 0 && left_fold<T>(op)) shape = 2;
   // shapes: 0 = look-back warp, default tile; 1 = warp 0 runs the look-back,
   // default tile; 2 = look-back warp, 64 KB tiles
   const uint64_t tile_items = !smem_path ? ScanCfg<T>::TILE
@@ -627,8 +634,9 @@ int scan_entry(mb_executor* ex, const mb_src* in, int op, bool exclusive, const 
 // look-back scratch (tile ticket, abort word, tile states) lives in this
 // fixed array instead of the executor's pool.  The largest call it admits
 // is 2^26 8-byte elements on the register-tiled path: 32,768 tiles, whose
-// states take 655,616 bytes, plus two group-state arrays of 12,544 bytes
-// and the 256-byte header, 680,960 bytes in all; the array is 1 MiB.  The
+// states take 655,616 bytes, plus two group-state arrays of 12,544 bytes,
+// the groups' lines of 131,200 bytes and the 256-byte header, 812,160 bytes in
+// all; the array is 1 MiB.  The
 // code checks the exact size of every call against the array.
 constexpr size_t kNoAllocBytes = 1u << 20;
 constexpr uint64_t kNoAllocMax4 = 1ull << 27;  // 4-byte elements
@@ -672,7 +680,9 @@ int scan_noalloc_run(mb_executor* ex, const mb_src& in, int op, const mb_col& ou
   const bool plain = src_plain(in, DTypeOf<T>::value) && out.dtype == DTypeOf<T>::value &&
                      ((uintptr_t)in.data % 16 == 0) && ((uintptr_t)out.data % 16 == 0);
   const bool smem_path = plain && in.len_dev == nullptr;
-  const uint64_t tile_items = smem_path ? SmemCfg<T>::TILE : ScanCfg<T>::TILE;
+  const bool big = left_fold<T>(op);
+  const uint64_t tile_items =
+      !smem_path ? ScanCfg<T>::TILE : big ? BigCfg<T>::TILE : SmemCfg<T>::TILE;
   const uint64_t tiles = (cap + tile_items - 1) / tile_items;
   const size_t state_bytes = TileState<T, PACKED>::bytes(tiles);
   const size_t need = 256 + state_bytes + GroupLines<T>::bytes(tiles);
@@ -694,15 +704,16 @@ int scan_noalloc_run(mb_executor* ex, const mb_src& in, int op, const mb_col& ou
   p.lines.base = (char*)scratch + 256 + state_bytes;
   const Src s = to_src(in);
   dim3 grid(grid_for(tiles)), block(kThreads);
-  const size_t smem = SmemCfg<T>::TILE_BYTES;
+  const size_t smem = big ? BigCfg<T>::TILE_BYTES : SmemCfg<T>::TILE_BYTES;
 #define MB_SCAN_NOALLOC_LAUNCH(OPID)                                                            \
   do {                                                                                          \
     if (smem_path) {                                                                            \
+      auto kern = big ? scan_smem_lb_kernel<T, OPID, PACKED, BigCfg<T>>                         \
+                      : scan_smem_lb_kernel<T, OPID, PACKED, SmemCfg<T>>;                       \
       if (smem > 48 * 1024)                                                                     \
-        MB_CUDA(cudaFuncSetAttribute(scan_smem_lb_kernel<T, OPID, PACKED, SmemCfg<T>>,          \
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));  \
-      scan_smem_lb_kernel<T, OPID, PACKED, SmemCfg<T>>                                          \
-          <<<grid, kThreads + 32, smem, ex->stream>>>((const T*)in.data, (T*)out.data, cap, p,  \
+        MB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,         \
+                                     (int)smem));                                               \
+      kern<<<grid, kThreads + 32, smem, ex->stream>>>((const T*)in.data, (T*)out.data, cap, p,  \
                                                       st);                                      \
     } else if (plain) {                                                                         \
       scan_kernel<T, OPID, true, PACKED><<<grid, block, 0, ex->stream>>>(s, out.data, cap, p, st); \

@@ -125,6 +125,8 @@ __global__ void __launch_bounds__(kBlock)
     flags[t] = (e.start ? 1 : 0) | (e.any ? 2 : 0);
   }
   if (threadIdx.x == 0) {
+    // A single block has none before it: what the top kernel would leave.
+    if (gridDim.x == 1) all = Fold<V>{V(0), false, false};
     top[blockIdx.x] = all.v;
     topf[blockIdx.x] = (all.start ? 1 : 0) | (all.any ? 2 : 0);
   }
@@ -264,8 +266,10 @@ int carry_run(mb_executor* ex, const CarryShape& s, int op, int exclusive, const
   seg_carry_blocks_kernel<V><<<(unsigned)blocks, kBlock, 0, ex->stream>>>(
       s, op, (const V*)part_tail, carry, flags, top, topf);
   MB_CUDA(cudaGetLastError());
-  seg_carry_top_kernel<V><<<1, kBlock, 0, ex->stream>>>(blocks, op, top, topf);
-  MB_CUDA(cudaGetLastError());
+  if (blocks > 1) {
+    seg_carry_top_kernel<V><<<1, kBlock, 0, ex->stream>>>(blocks, op, top, topf);
+    MB_CUDA(cudaGetLastError());
+  }
   V i;
   memcpy(&i, init, sizeof(V));
 #define MB_CARRY_OUT(OUT) \
