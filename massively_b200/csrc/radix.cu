@@ -52,6 +52,7 @@ constexpr int kRadixBits = 8;
 constexpr int kBins = 1 << kRadixBits;
 constexpr int kHistThreads = 512;
 constexpr int kHistUnroll = 4;  // 16-byte vectors per lane per chunk
+constexpr uint32_t kMixItems = 1u << 25;  // see ballot_round
 
 // Look-back status word of one (tile, digit): the flag (none / aggregate /
 // inclusive) in the top two bits, the digit's count below.  32-bit words
@@ -580,19 +581,25 @@ struct OnesweepTmaSmem {
   uint64_t bar;
 };
 
-// Rounds that find their peers by ballots although a mask table is there (one
-// table).  The mask table's three accesses per round are what fills the
-// shared-memory pipe, the ballots' logic what fills the ALU pipe, so a mix
-// loads both: 2^28 u32 pairs 6.38 ms with masks alone, 6.71 ms with ballots
-// alone, 6.10 / 6.07 / 6.31 ms with 4 / 8 / 12 of 16 rounds by ballots; 40 M
-// Zipf(1.1) pairs (few digits, many peers) 1.25 -> 1.08 ms.  64-bit keys,
-// 2^25: 1.86 / 1.77 / 1.78 / 1.89 ms with 0 / 4 / 8 / 12 rounds.
+// Rounds of a mixed pass that find their peers by ballots although a mask
+// table is there (one table).  The mask table's three accesses per round are
+// what fills the shared-memory pipe, the ballots' logic what fills the ALU
+// pipe, so a mix loads both: 2^28 u32 pairs 6.38 ms with masks alone, 6.71 ms
+// with ballots alone, 6.10 / 6.07 / 6.31 ms with 4 / 8 / 12 of 16 rounds by
+// ballots; 40 M Zipf(1.1) pairs (few digits, many peers) 1.25 -> 1.08 ms.
+// Uniform columns that stay in L2 gain nothing (6 M pairs 235 -> 241 us), so
+// 4-byte keys mix from kMixItems items (the capacity: a device length is not
+// known here).  Both forms in one kernel, chosen per pass on the device, cost
+// the large sorts what the mix gains (6.29 ms).  64-bit keys always mix: 2^22 -
+// 3 keys 337 -> 320 us, 2^25 1.86 / 1.77 / 1.78 / 1.89 ms with 0 / 4 / 8 / 12
+// rounds.
 template <class K>
 __device__ constexpr bool ballot_round(int k) {
   return k % 4 < (sizeof(K) == 4 ? 2 : 1);
 }
 
-template <class K, int ENC, class V, int THREADS, int ITEMS, int NT, bool P64, bool FULL, class SW>
+template <class K, int ENC, class V, int THREADS, int ITEMS, int NT, bool P64, bool FULL, bool MIX,
+          class SW>
 __device__ __forceinline__ void onesweep_tile(OnesweepTmaSmem<K, V, THREADS, ITEMS, NT>& sm,
                                               const uint32_t tile, const uint32_t valid,
                                               const int pass, const uint32_t n,
@@ -657,7 +664,7 @@ __device__ __forceinline__ void onesweep_tile(OnesweepTmaSmem<K, V, THREADS, ITE
       const uint32_t d =
           (FULL || li < valid) ? digit_of<K, ENC>(sm.keys[li], shift) : (uint32_t)kBins;
       rd[k] = d << 16;
-      if constexpr (NT == 1) {
+      if constexpr (MIX) {
         if (ballot_round<K>(k)) {
           constexpr int NB = FULL ? kRadixBits : kRadixBits + 1;
           uint32_t eq = kFull;
@@ -817,7 +824,8 @@ __device__ __forceinline__ void onesweep_tile(OnesweepTmaSmem<K, V, THREADS, ITE
 
 // MINB: CTAs per SM the registers are budgeted for (0 = by tile shape);
 // SW: the look-back status word (DigitStatus).
-template <class K, int ENC, class V, int THREADS, int ITEMS, int NT, bool P64, int MINB, class SW>
+template <class K, int ENC, class V, int THREADS, int ITEMS, int NT, bool P64, int MINB, bool MIX,
+          class SW>
 __global__ void __launch_bounds__(THREADS, MINB > 0 ? MINB
                                           : NT <= 1 ? (THREADS >= 1024 ? 1 : THREADS >= 384 ? 2 : 4)
                                                     : 3)
@@ -879,18 +887,16 @@ __global__ void __launch_bounds__(THREADS, MINB > 0 ? MINB
   V* out_v = (V*)plan->out_v[pass];
   if (valid == TILE) {
     if (!mbar_wait(&sm.bar, 0)) raise_device_error(err, MB_DEV_ERR_LOOKBACK);
-    onesweep_tile<K, ENC, V, THREADS, ITEMS, NT, P64, true, SW>(sm, tile, valid, pass, n,
-                                                               digit_offsets, status, err, out_k,
-                                                               out_v);
+    onesweep_tile<K, ENC, V, THREADS, ITEMS, NT, P64, true, MIX, SW>(
+        sm, tile, valid, pass, n, digit_offsets, status, err, out_k, out_v);
   } else {
     for (uint32_t i = tid; i < valid; i += THREADS) {
       sm.keys[i] = in_k[tile_base + i];
       if constexpr (!KEYS_ONLY) sm.vals[i] = in_v[tile_base + i];
     }
     __syncthreads();
-    onesweep_tile<K, ENC, V, THREADS, ITEMS, NT, P64, false, SW>(sm, tile, valid, pass, n,
-                                                                digit_offsets, status, err, out_k,
-                                                                out_v);
+    onesweep_tile<K, ENC, V, THREADS, ITEMS, NT, P64, false, MIX, SW>(
+        sm, tile, valid, pass, n, digit_offsets, status, err, out_k, out_v);
   }
 }
 
@@ -981,8 +987,13 @@ int onesweep_sort_cfg(mb_executor* ex, const K* in_k, const V* in_v, K* out_k, V
                        (KEYS_ONLY || ((uintptr_t)in_v % 16 == 0 && (uintptr_t)out_v % 16 == 0));
   if (aligned) {
     const size_t smem = sizeof(OnesweepTmaSmem<K, V, THREADS, ITEMS, NT>);
-    auto kern = radix_onesweep_tma_kernel<K, ENC, V, THREADS, ITEMS, NT,
-                                          P64 && sizeof(K) == 4 && sizeof(V) == 4, MINB, SW>;
+    constexpr bool PAIR64 = P64 && sizeof(K) == 4 && sizeof(V) == 4;
+    constexpr bool CHOOSE = NT == 1 && sizeof(K) == 4;
+    auto kern = radix_onesweep_tma_kernel<K, ENC, V, THREADS, ITEMS, NT, PAIR64, MINB,
+                                          NT == 1 && sizeof(K) == 8, SW>;
+    if constexpr (CHOOSE)
+      if (n >= kMixItems)
+        kern = radix_onesweep_tma_kernel<K, ENC, V, THREADS, ITEMS, NT, PAIR64, MINB, true, SW>;
     MB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     for (int p = 0; p < PASSES; ++p) {
       {
