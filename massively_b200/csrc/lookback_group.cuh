@@ -127,8 +127,12 @@ __device__ __forceinline__ T lookback_two_level(const State& st, const GroupLine
     if (lane == 0) st.gagg.publish((uint64_t)g, a);
   }
   if (g == 0) return hs;
+  // Every lane polls the same word, but two lanes' loads may still see
+  // different values for a while: the exit is voted.
   T acc = fallback;
-  while (!lines.peek((uint64_t)g, acc)) {  // the same word for every lane
+  while (true) {
+    const bool seen = lines.peek((uint64_t)g, acc);
+    if (__all_sync(kFull, seen)) break;
     __nanosleep(kPollSleepNs);
     if (__any_sync(kFull, guard.expired())) {
       raise_device_error(err, MB_DEV_ERR_LOOKBACK);
