@@ -173,12 +173,13 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
   }
 
-  if (out_k)
-    for (uint32_t i = tid; i < n; i += kThreads) out_k[i] = small_dec<K>(sm.key[i], enc);
+  // Values before keys: out_k may be the value column (in_k is not read again).
   if (vsize == 4)
     small_gather<uint32_t>(sm, (const uint32_t*)in_v, (uint32_t*)out_v, n);
   else if (vsize == 8)
     small_gather<uint64_t>(sm, (const uint64_t*)in_v, (uint64_t*)out_v, n);
+  if (out_k)
+    for (uint32_t i = tid; i < n; i += kThreads) out_k[i] = small_dec<K>(sm.key[i], enc);
 }
 
 template <class K, int ITEMS>

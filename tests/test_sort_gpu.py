@@ -276,3 +276,18 @@ def test_radix_sort_beyond_2e30_items(ex):
     seen = torch.zeros(n, dtype=torch.int8, device=v.device)
     seen[v] = 1
     assert bool(seen.all()), "values are not a permutation"
+
+
+@pytest.mark.parametrize("n", [3001, 16384, 20_000])
+def test_pairs_into_each_others_columns(ex, n):
+    """Sorted keys written to the value column and values to the key column."""
+    from massively_b200 import _native as N
+    from massively_b200.runtime import check
+    keys, vals = seeded(np.uint32, n, 31), seeded(np.uint32, n, 32)
+    perm = orc.radix_perm([keys])
+    a, b = ex.to_device(keys), ex.to_device(vals)
+    check(N.lib().mb_radix_sort_by_key(ex.handle, (N.mb_src * 1)(a.to_src()), 1,
+                                       (N.mb_src * 1)(b.to_src()), 1, (N.mb_col * 1)(a.to_col()),
+                                       (N.mb_col * 1)(b.to_col())))
+    np.testing.assert_array_equal(ex.to_host(b), keys[perm])
+    np.testing.assert_array_equal(ex.to_host(a), vals[perm])
