@@ -927,6 +927,12 @@ bool window_order(const mb_src& l, const mb_src& r, int less, bool ties, int& en
   return true;
 }
 
+// Whether `out` shares memory with the column `in` (`bytes` of each).
+inline bool overlaps(const void* out, const mb_src& in, uint64_t bytes) {
+  const uintptr_t o = (uintptr_t)out, i = (uintptr_t)in.data;
+  return o < i + bytes && i < o + bytes;
+}
+
 inline bool aligned16(const mb_src& l, const mb_src& r) {
   return (uintptr_t)l.data % 16 == 0 && (uintptr_t)r.data % 16 == 0;
 }
@@ -1065,7 +1071,11 @@ int set_run(mb_executor* ex, const mb_src& l, const mb_src& r, int less, int mod
   using U = typename UnsignedOf<T>::type;
   int enc = 0;
   U flip = 0;
-  if (mode != 0 && window_order<T>(l, r, less, false, enc, flip)) {
+  // (The window kernel looks up run starts in left items of earlier tiles, the
+  // tile kernel reads only its own slice: an output over the left column is
+  // its business.)
+  if (mode != 0 && window_order<T>(l, r, less, false, enc, flip) &&
+      !overlaps(out.data, l, l.len * sizeof(T))) {
     if constexpr (std::is_floating_point<T>::value) {
       if (enc == 1) return set_window<U, 1>(ex, l, r, mode == 2, flip, out.data, count_dev);
       return set_window<U, 2>(ex, l, r, mode == 2, flip, out.data, count_dev);

@@ -140,3 +140,30 @@ def test_set_ops_device_length_and_lazy_inputs(ex):
     none = vector.copy_where(ex, ex.to_device(x[:10]), ex.to_device(np.zeros(10, np.uint32)))
     got = vector.set_union(ex, none, none)
     assert got.logical_len() == 0
+
+
+@pytest.mark.parametrize("mode", ["intersection", "difference"])
+def test_set_operation_into_its_left_column(ex, mode):
+    """A run far longer than what is in flight at a time, behind items that are dropped: the
+    output then covers items before the run's start while its later tiles still look for it."""
+    import ctypes as C
+
+    from massively_b200 import _native as N, vector
+    from massively_b200.runtime import check
+    run, front, lost = 1 << 23, 1 << 22, 1000
+    left = np.concatenate([np.arange(front, dtype=np.uint32),
+                           np.full(run, 0x7FFFFFFF, np.uint32)])
+    if mode == "intersection":
+        right = left[front + lost:]
+        want = right
+    else:
+        right = left[:front + lost]
+        want = left[front + lost:]
+    l, r = ex.to_device(left), ex.to_device(right)
+    cnt = vector._count_buffer(ex)
+    check(getattr(N.lib(), f"mb_set_{mode}")(
+        ex.handle, C.byref(l.to_src()), C.byref(r.to_src()), 0,  # MB_LESS
+        l.to_col(), vector._p32(cnt), None))
+    got = l.with_len_dev(cnt)
+    assert got.logical_len() == want.size
+    np.testing.assert_array_equal(ex.to_host(got)[:want.size], want)
