@@ -548,7 +548,8 @@ int mb_graph_destroy(mb_graph* graph);
  * one of the MB_TUNE_* ids; `config` is below mb_tune_config_count(family). */
 enum {
   MB_TUNE_SCAN = 0,
-  MB_TUNE_RADIX = 1,
+  MB_TUNE_RADIX = 1, /* onesweep passes; columns of at most 16384 4-byte or 8192 8-byte keys
+                        are sorted by one CTA instead, whatever is selected */
   MB_TUNE_REDUCE = 2,
   MB_TUNE_SELECT = 3,
   MB_TUNE_SEG = 4, /* ForEachSegment(Reduce): tile-local folds or a carried look-back */

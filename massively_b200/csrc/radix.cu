@@ -1117,9 +1117,9 @@ int bounded_wait_check(mb_executor* ex, int kind) {
 // the device by an earlier step; no host synchronisation).
 int radix_sort_plain(mb_executor* ex, int kdt, const void* ik, const void* iv, void* ok, void* ov,
                      size_t vsize, uint64_t n, const uint32_t* n_dev) {
-  // A column that fits one CTA (smallsort.cu), unless a shape was chosen.
-  if (ex->tune[MB_TUNE_RADIX] < 0 && wide_key(kdt) && (vsize == 0 || vsize == 4 || vsize == 8) &&
-      n <= small_sort_max(kdt))
+  // A column that fits one CTA (smallsort.cu), whatever shape the onesweep has
+  // been given: that choice was made for longer columns.
+  if (wide_key(kdt) && (vsize == 0 || vsize == 4 || vsize == 8) && n <= small_sort_max(kdt))
     return small_sort(ex, kdt, ik, iv, ok, ov, vsize, n, n_dev);
   switch (kdt) {
     case MB_U32: return sort_keys_vals<uint32_t, kEncUnsigned>(ex, ik, iv, ok, ov, vsize, n, n_dev);

@@ -6,7 +6,9 @@ include/massively_b200.h, listed by `mb_tune_config_count` /
 
 - radix: onesweep tile shape (threads per CTA, keys per thread), CTAs per
   SM, peer discovery (shared-memory lane masks or ballots) and 64-bit pair
-  staging; the digit width is 8 bits in every configuration;
+  staging; the digit width is 8 bits in every configuration (columns of at
+  most 16384 4-byte or 8192 8-byte keys are sorted by one CTA whatever is
+  selected);
 - scan: tile size and which warp runs the look-back;
 - seg: ForEachSegment(Reduce) as tile-local folds or a carried look-back;
 - reduce, select: one configuration each.

@@ -176,11 +176,19 @@ def test_every_radix_config_bit_exact(n, keyspace):
         keys = np.full(n, 3, np.uint32)
     vals = _perm_values(n)
     want = orc.radix_perm([keys])
+    # Columns of at most 16384 rows would be sorted by one CTA whatever the
+    # configuration: the rows lie in a longer column with a device length.
+    pad = np.zeros(max(0, 20_000 - n), np.uint32)
+    count = ex.to_device(np.array([n], np.uint32)).tensor if pad.size else None
+
+    def column(x):
+        return ex.to_device(np.concatenate([x, pad.view(x.dtype)])).with_len_dev(count)
+
     for cfg in range(len(tune.configs("radix"))):
         tune.set_config(ex, "radix", cfg)
         for kdt in (np.uint32, np.float32):
             k = keys.view(kdt)
-            sk, sv = vector.radix_sort_pairs(ex, ex.to_device(k), ex.to_device(vals))
+            sk, sv = vector.radix_sort_pairs(ex, column(k), column(vals))
             w = want if kdt == np.uint32 else orc.radix_perm([k])
             np.testing.assert_array_equal(ex.to_host(sv), w, err_msg=f"config {cfg} {kdt}")
     ex.sync()
@@ -212,6 +220,54 @@ def test_kernel_timing_counts_onesweep_launches():
     cnt = C.c_uint64()
     L.mb_kernel_timing_read(ex.handle, N.KF_RADIX_ONESWEEP, C.byref(cnt), None)
     assert cnt.value == 0  # read forgets
+
+
+def _onesweep_launches(ex, run):
+    import ctypes as C
+
+    from massively_b200 import _native as N
+    cnt = C.c_uint64()
+    N.lib().mb_kernel_timing_read(ex.handle, N.KF_RADIX_ONESWEEP, None, None)
+    N.lib().mb_kernel_timing(ex.handle, 1)
+    run()
+    N.lib().mb_kernel_timing(ex.handle, 0)
+    assert N.lib().mb_kernel_timing_read(ex.handle, N.KF_RADIX_ONESWEEP, C.byref(cnt), None) == 0
+    return cnt.value
+
+
+@pytest.mark.parametrize("dtype,top", [(np.uint32, 16384), (np.int64, 8192)])
+def test_small_sorts_take_no_passes_under_a_chosen_shape(dtype, top):
+    """A shape chosen for the onesweep passes leaves the columns that one CTA sorts with one
+    launch."""
+    from massively_b200 import tune, vector
+    ex = executor()
+    passes = {top: 0, top + 1: np.dtype(dtype).itemsize}
+    for n, want in passes.items():
+        k, v = ex.to_device(seeded(dtype, n, 1)), ex.to_device(_perm_values(n))
+        for cfg in (-1, 0, 2):
+            tune.set_config(ex, "radix", cfg)
+            assert _onesweep_launches(ex, lambda: vector.radix_sort_pairs(ex, k, v)) == want
+    ex.sync()
+
+
+def test_small_sorts_take_no_passes_after_tuning(tmp_path):
+    """... and so do a shape tuned on a small column and one recorded for a longer one."""
+    from massively_b200 import tune, vector
+    ex = executor()
+    db = str(tmp_path / "tune.json")
+    cols = {n: (ex.to_device(seeded(np.uint32, n, 1)), ex.to_device(_perm_values(n)))
+            for n in (3001, 100_000)}
+
+    def run(n):
+        return lambda: vector.radix_sort_pairs(ex, *cols[n])
+
+    for n in (100_000, 3001):
+        tune.autotune(ex, "radix", "u32", n, run(n), reps=1, warmup=1, path=db)
+        assert _onesweep_launches(ex, run(3001)) == 0
+    assert tune.apply(ex, "u32", 100_000, path=db)["radix"][1] == "db"
+    assert _onesweep_launches(ex, run(3001)) == 0
+    assert _onesweep_launches(ex, run(100_000)) == 4
+    ex.sync()
 
 
 def test_autotune_records_and_selects_fastest(tmp_path):
