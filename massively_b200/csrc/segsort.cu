@@ -11,10 +11,10 @@
 //     segments longer than a tile.
 //   * One CTA per range sorts the range's segments no longer than kSsRange as
 //     one pack -- fewer than kSsTile items, since the last of them starts
-//     inside the range -- by (segment within the pack, encoded value) with a
-//     stable LSD radix sort of 8-bit digits in shared memory.  A digit that
-//     is the same for every item of the pack is skipped, so a pack of one
-//     segment takes four passes and a pack of up to 256 segments five.  A
+//     inside the range -- by one word of (segment within the pack, encoded
+//     value) with a stable LSD radix sort of 8-bit digits in shared memory:
+//     three passes over the word's top 24 bits where few items agree there,
+//     else over the digits that vary (ss_pack).  A
 //     longer segment can only be the range's last one (it reaches past the
 //     range); it is sorted next by the same CTA when it fits a tile.
 //   * Segments longer than a tile go to the first CTAs of the same grid, one
@@ -54,14 +54,30 @@ constexpr int kSsTile = kSsThreads * kSsItems;  // 4096 items
 constexpr int kSsRange = kSsTile / 2;           // 2048 start positions per range
 constexpr int kSsBins = 256;
 constexpr int kSsWordBits = 24;                 // of (segment, value) that a pack sorts by passes
+// Threads that may hold close neighbours where bits are left out, times the
+// pack's mean segment length: above it the items that would agree cost more to
+// order afterwards than a pass more (ss_pack).  2^24 u32 below 2^20 with outliers
+// in segments of 64 / 256 items, 32 / 128 agreeing neighbours to a pack: three
+// passes 480 / 496 us, four 463 / 467 us.  The look itself costs 1% of a sort of
+// uniform words.
+constexpr uint32_t kSsTies = 1024;
 constexpr int kSsNT = 3;                        // lane-mask tables used in turn
 constexpr uint32_t kSsLongLimit = 1u << 17;     // longest segment one CTA sorts
 constexpr uint32_t kSsLongCtas = 2 * 148;
 static_assert(kSsThreads == kSsBins, "one thread per digit in the digit scans");
 
+// How a pack is sorted (ss_pack); in shared memory, since the passes leave no
+// registers for it.
+struct SsPlan {
+  uint32_t every, todo;  // passes, one bit per digit: by all varying digits, and the ones taken
+  uint32_t low;          // value bits left out
+  uint32_t least;        // taken off every value
+  int up, off;           // bits of a key below its segment, bits below its first digit
+};
+
 template <bool PAY>
 struct SsSmem {
-  uint64_t keys[kSsTile];  // (segment within the pack << 32) | encoded value
+  uint64_t keys[kSsTile];  // segment within the pack above the encoded value (ss_pack)
   uint32_t pay[PAY ? kSsTile : 1];
   uint32_t mask[kSsNT][kSsWarps][kSsBins];
   uint32_t warp_cnt[kSsWarps][kSsBins];
@@ -72,8 +88,9 @@ struct SsSmem {
   uint32_t heads[kSsTile / 32];  // segment starts in the pack, one bit per item
   uint32_t hpre[kSsTile / 32];   // starts in the words before
   uint32_t wsum[kSsWarps];
-  uint32_t red[kSsWarps][4];
+  uint32_t red[kSsWarps][3];     // bits that differ, least and greatest value
   uint32_t flag[4];
+  SsPlan plan;
 };
 
 template <int ENC>
@@ -326,108 +343,131 @@ __device__ __forceinline__ void ss_pack(SsSmem<PAY>& sm, const Src& in, const ui
     if (tid < kSsTile / 32) sm.hpre[tid] = ex;
   }
   __syncthreads();
-  // Which value bits differ between some two items.
-  uint32_t or_lo = 0, and_lo = ~0u;
+  // The values' range, and which of their bits differ between some two items.
+  const uint32_t ref = ss_encode<ENC>(raw[0], desc, ieee);
+  uint32_t var = 0, lo = ~0u, hi = 0;
 #pragma unroll
   for (int k = 0; k < kSsItems; ++k) {
     if ((uint32_t)k * kSsThreads + tid < len) {
       const uint32_t u = ss_encode<ENC>(raw[k], desc, ieee);
-      or_lo |= u;
-      and_lo &= u;
+      var |= u ^ ref;
+      lo = min(lo, u);
+      hi = max(hi, u);
     }
   }
-  or_lo = __reduce_or_sync(kFull, or_lo);
-  and_lo = __reduce_and_sync(kFull, and_lo);
+  lo = __reduce_min_sync(kFull, lo);
+  hi = __reduce_max_sync(kFull, hi);
+  if ((uint32_t)tid < len) var |= ref ^ lo;
+  var = __reduce_or_sync(kFull, var);
   if (lane == 0) {
-    sm.red[warp][0] = or_lo;
-    sm.red[warp][1] = and_lo;
+    sm.red[warp][0] = var;
+    sm.red[warp][1] = lo;
+    sm.red[warp][2] = hi;
   }
   __syncthreads();
-  uint32_t var_lo, same;
   {
-    uint32_t a = 0, b = ~0u;
-#pragma unroll
-    for (int w = 0; w < kSsWarps; ++w) {
-      a |= sm.red[w][0];
-      b &= sm.red[w][1];
-    }
-    var_lo = a ^ b;
-    same = b;  // the value bits outside var_lo
+    const bool on = lane < kSsWarps && (uint32_t)lane * 32 < len;  // a warp with items
+    const uint32_t l = on ? sm.red[lane][1] : ~0u;
+    hi = __reduce_max_sync(kFull, on ? sm.red[lane][2] : 0u);
+    lo = __reduce_min_sync(kFull, l);
+    var = __reduce_or_sync(kFull, on ? sm.red[lane][0] | (l ^ lo) : 0u);
   }
   const uint32_t nseg =
       sm.hpre[kSsTile / 32 - 1] + (uint32_t)__popc(sm.heads[kSsTile / 32 - 1]);
-  const int vb = 32 - __clz(var_lo), sb = nseg > 1 ? 32 - __clz(nseg - 1) : 0;
-
-  // The keys of the passes: segment within the pack above the value, of which
-  // only the bits up to the highest varying one count, so that the two lie
-  // together; and of that word only the top 24 bits are sorted, in three
-  // passes, where sorting the varying digits of segment and value one by one
-  // would take more.  ss_fix_runs then orders the runs that agree there: a
-  // segment of a few hundred items rarely has any.  (2^26 u32 in 2^20
-  // segments: 1.59 -> 1.40 ms; with 16 bits 1.36 ms, but then floats, whose top bits are
-  // exponents, leave long runs.)  Otherwise the lowest of four varying value
-  // digits is left out in the same way: a pack's keys rarely agree on segment
-  // and the value's top three digits.  (Leaving out two digits saved a pass
-  // but made runs common enough that their fix-up cost more.)
-  uint32_t low = 0;  // the value bits left out
-  int digits = (sb + 7) / 8;
-  {
-    int m = 0, c = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) m += ((var_lo >> (8 * j)) & 0xFFu) != 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (((var_lo >> (8 * j)) & 0xFFu) && ++c == m - 3)
-        low = j == 3 ? ~0u : ((1u << (8 * j + 8)) - 1u);
-    digits += m > 3 ? 3 : m;
-  }
-  static_assert(kSsTile <= 1 << 12, "a pack's segment numbers leave 12 bits of the word");
-  const int drop = max(0, sb + vb - kSsWordBits);
-  bool packed = (sb + vb - drop + 7) / 8 < digits;
-  if (packed) low = drop ? (1u << drop) - 1u : 0u;
-  const int up = packed ? vb : 32;
-  uint32_t vmask = up == 32 ? ~0u : (1u << up) - 1u;  // the value bits held in the key
   auto segment_of = [&](uint32_t p) -> uint32_t {
     const uint32_t w = p >> 5;
     return sm.hpre[w] + (uint32_t)__popc(sm.heads[w] & (0xFFFFFFFFu >> (31 - (p & 31)))) - 1u;
   };
+
+  // The keys of the passes: segment within the pack above the value less the
+  // pack's least, of which only the bits of the range count, so that the two
+  // lie together; and of that word only the top 24 bits are sorted, in three
+  // passes, where sorting the varying digits of segment and value one by one
+  // would take more.  ss_fix_runs then orders the runs that agree there.
+  // (2^26 u32 in 2^20 segments: 1.59 -> 1.40 ms; with 16 bits 1.36 ms, but then
+  // floats, whose top bits are exponents, leave long runs.)  Otherwise the
+  // lowest of four varying value digits is left out in the same way.  (Leaving
+  // out two digits saved a pass but made runs common enough that their fix-up
+  // cost more.)
+  static_assert(kSsTile <= 1 << 12, "a pack's segment numbers leave 12 bits of the word");
+  uint32_t every, todo;   // passes, one bit per digit: by all varying digits, and the ones taken
+  uint32_t low;           // value bits left out
+  int up = 32, off0 = 0;  // bits of a key below its segment, bits below the first digit
+  {
+    const int vb = 32 - __clz(hi - lo), sb = nseg > 1 ? 32 - __clz(nseg - 1) : 0;
+    every = ((1u << ((sb + 7) / 8)) - 1u) << 4;
 #pragma unroll
-  for (int k = 0; k < kSsItems; ++k) {
-    const uint32_t p = (uint32_t)k * kSsThreads + tid;
-    if (p < len) {
-      sm.keys[p] = ((uint64_t)segment_of(p) << up) | (ss_encode<ENC>(raw[k], desc, ieee) & vmask);
-      if constexpr (PAY) sm.pay[p] = raw[k];
+    for (int j = 0; j < 4; ++j) every |= ((var >> (8 * j)) & 0xFFu) != 0 ? 1u << j : 0u;
+    low = (every & 15u) == 15u ? 0xFFu : 0u;
+    todo = every & ~(low & 1u);
+    const int drop = max(0, sb + vb - kSsWordBits), word = (sb + vb - drop + 7) / 8;
+    if (word < __popc(todo)) {
+      low = (1u << drop) - 1u;
+      todo = (1u << word) - 1u;
+      up = vb;
+      off0 = drop;
+    } else {
+      lo = 0;
     }
   }
-  __syncthreads();
   while (true) {
-    for (int pass = 0; pass < 8; ++pass) {
-      int shift = 8 * pass;
-      if (packed) {
-        shift += drop;
-        if (shift >= sb + vb) break;
-      } else if (shift < 32 ? !((var_lo & ~low) >> shift & 0xFFu) : shift - 32 >= sb) {
-        continue;
+#pragma unroll
+    for (int k = 0; k < kSsItems; ++k) {
+      const uint32_t p = (uint32_t)k * kSsThreads + tid;
+      if (p < len) {
+        sm.keys[p] = ((uint64_t)segment_of(p) << up) | (ss_encode<ENC>(raw[k], desc, ieee) - lo);
+        if constexpr (PAY) sm.pay[p] = raw[k];
       }
-      ss_pass(sm, len, shift);
     }
-    if (!low || ss_fix_runs(sm, len, low)) break;
+    // Bits are left out only where few items of a segment would then agree: a
+    // range that one outlier, or a heavy tail, sets apart leaves all the others
+    // in one run, which would have to be sorted again.  Looked at are the
+    // neighbours in two rounds that differ, but by no more than those bits; if
+    // they are many, only the lowest digit is left out, and then nothing.  (2^24
+    // i32 in +-4096 in segments of 256: 247 us, 855 us with bits taken from the
+    // highest one that differs; u32 below 4096 with an outlier in 1500: 526 and
+    // 863 us.)
+    bool close = false;
+#pragma unroll
+    for (int k = 0; k < 8; k += 4) {
+      const uint32_t u = ss_encode<ENC>(raw[k], desc, ieee);
+      const uint32_t v = __shfl_down_sync(kFull, u, 1);
+      if ((uint32_t)k * kSsThreads + tid + 1 < len && lane < 31)
+        close |= max(u, v) - min(u, v) - 1u < low;
+    }
+    if (tid == 0) {
+      sm.plan.todo = todo;
+      sm.plan.every = every;
+      sm.plan.low = low;
+      sm.plan.up = up;
+      sm.plan.off = off0;
+      sm.plan.least = lo;
+    }
+    if ((uint32_t)__syncthreads_count(close) * len <= kSsTies * nseg) break;
+    low = up < 32 || off0 > 0 ? ((every & 15u) == 15u ? 0xFFu : 0u) : 0u;
+    todo = every & ~(low & 1u);
+    up = 32;
+    off0 = 0;
+    lo = 0;
+  }
+  while (true) {
+    for (int j = 0; j < 8; ++j)
+      if ((sm.plan.todo >> j) & 1u) ss_pass(sm, len, sm.plan.off + 8 * j);
+    if (!sm.plan.low || ss_fix_runs(sm, len, sm.plan.low)) break;
     // A long run out of order: build the keys again and take every digit.
     for (uint32_t p = tid; p < len; p += kSsThreads) {
       const uint32_t r = ss_load<PLAIN>(in, (uint64_t)start + p);
       sm.keys[p] = ((uint64_t)segment_of(p) << 32) | ss_encode<ENC>(r, desc, ieee);
       if constexpr (PAY) sm.pay[p] = r;
     }
+    if (tid == 0) sm.plan = SsPlan{sm.plan.every, sm.plan.every, 0u, 0u, 32, 0};
     __syncthreads();
-    packed = false;
-    low = 0;
-    vmask = ~0u;
   }
-  same &= ~vmask;
+  const uint32_t vmask = sm.plan.up == 32 ? ~0u : (1u << sm.plan.up) - 1u, least = sm.plan.least;
   for (uint32_t p = tid; p < len; p += kSsThreads) {
     uint32_t v;
     if constexpr (PAY) v = sm.pay[p];
-    else v = ss_decode<ENC>(((uint32_t)sm.keys[p] & vmask) | same, desc);
+    else v = ss_decode<ENC>(((uint32_t)sm.keys[p] & vmask) + least, desc);
     out[(uint64_t)start + p] = v;
   }
   __syncthreads();  // shared memory is reused by the next pack

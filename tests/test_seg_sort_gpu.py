@@ -198,3 +198,60 @@ def test_runs_equal_in_the_high_digits(ex, less):
     f[np.isnan(f)] = np.float32(-0.0)
     got = _run(ex, f, off, less)
     assert np.array_equal(got.view(np.uint32), orc.seg_sort(f, off, less).view(np.uint32))
+
+
+def _narrow(kind, n):
+    """Values of both signs around zero; small values behind one outlier per 1500 items; a heavy
+    tail (few values far above the others)."""
+    u = seeded(np.uint32, n, 77)
+    if kind == "signed":
+        return (u % np.uint32(8192)).astype(np.int32) - np.int32(4096)
+    if kind == "outlier":
+        x = u % np.uint32(4096)
+        x[::1500] = 0xFFFFFFFF
+        return x
+    if kind == "floats":
+        return ((u % np.uint32(8192)).astype(np.float32) - np.float32(4096)) / np.float32(4)
+    return np.minimum(((u.astype(np.float64) + 1) / 2.0 ** 32) ** -2, 2e9).astype(np.uint32)
+
+
+@pytest.mark.parametrize("kind", ["signed", "outlier", "tail", "floats"])
+@pytest.mark.parametrize("length", [5, 40, 256, 2000, 4096])
+@pytest.mark.parametrize("less", ["less", "greater"])
+def test_values_close_together(ex, kind, length, less):
+    from massively_b200 import op, seg
+    n = 20_011
+    x = _narrow(kind, n)
+    off = np.append(np.arange(0, n, length), n).astype(np.uint32)
+    s = seg.Segmentation.from_offsets(ex, ex.to_device(off))
+    got = seg.ForEachSegment(seg.Sort(op.pred2(less))).run(ex, s.segments(ex.to_device(x)))
+    np.testing.assert_array_equal(ex.to_host(got.values()).view(np.uint32),
+                                  orc.seg_sort(x, off, less).view(np.uint32))
+
+
+def test_values_close_together_are_sorted_once(ex):
+    """A pack is sorted in three to five passes.  Three that turn out not to do, and all of them
+    after that, are eight and a second read: more than twice the time of three, where five are
+    less than twice."""
+    import ctypes as C
+
+    from massively_b200 import _native as N, op, seg
+    seg_sort = 5  # MB_KF_SEG_SORT
+    n = 1 << 23
+    off = ex.to_device(np.arange(0, n + 1, 256).astype(np.uint32))
+    s = seg.Segmentation.from_offsets(ex, off)
+    ms = {}
+    for kind, x in [("uniform", seeded(np.uint32, n, 76)), ("signed", _narrow("signed", n)),
+                    ("outlier", _narrow("outlier", n))]:
+        it = s.segments(ex.to_device(x))
+        best = np.inf
+        for rep in range(8):
+            t = C.c_double()
+            N.lib().mb_kernel_timing(ex.handle, 1)
+            seg.ForEachSegment(seg.Sort(op.Less)).run(ex, it)
+            N.lib().mb_kernel_timing(ex.handle, 0)
+            N.lib().mb_kernel_timing_read(ex.handle, seg_sort, None, C.byref(t))
+            best = min(best, t.value)
+        ms[kind] = best
+    assert ms["uniform"] > 0
+    assert ms["signed"] < 1.8 * ms["uniform"] and ms["outlier"] < 1.8 * ms["uniform"], ms
