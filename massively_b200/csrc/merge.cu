@@ -528,14 +528,17 @@ __device__ __forceinline__ U ord_to_raw(U u, U flip) {
 }
 
 // The merge-path split of every tile boundary by groups of G lanes, G + 1
-// sub-ranges per round.  Lists that stay in L2 take eight lanes: a 27-step
-// binary search becomes nine rounds of independent loads, and the searches'
-// latency is what the tile kernel waits for.  Longer lists take two (17
-// rounds): the probes are random DRAM reads, and wide rounds make more of them
-// (100000007 + 150000001 u32 merged in 523 / 510 / 496 us with 8 / 4 / 2 lanes,
-// 7000000 + 9000000 in 49 / 54 / 54 us).  Boundaries past the logical end are
-// not computed.
-constexpr uint64_t kSplitWideItems = 1ull << 26;
+// sub-ranges per round.  Shorter lists take eight lanes: a 27-step binary search
+// becomes nine rounds of independent loads, and the searches' latency is what
+// the tile kernel waits for.  Longer ones take two (17 rounds): the probes are
+// then mostly DRAM reads, and wide rounds make more of them.  The line lies
+// between 64 and 80 M items of 4 bytes (merge 138.9 / 140.9 us with 8 / 2 lanes,
+// then 171.7 / 170.7; 265 / 258 us at 128 M) and between 32 and 48 M items of 8
+// (157.5 / 159.5, then 230.5 / 226.9; 301 / 295 us at 64 M), about twice the L2
+// cache.  It goes by capacity, a device length is not known here; two lanes cost
+// up to 5 us (16 M items of 4 bytes: 48.1 and 53.0 us).  Boundaries past the
+// logical end are not computed.
+constexpr uint64_t kSplitWideBytes = 1ull << 28;
 
 template <class U, int ENC, int G>
 __global__ void __launch_bounds__(kThreads)
@@ -940,7 +943,7 @@ inline bool aligned16(const mb_src& l, const mb_src& r) {
 template <class U, int ENC>
 int window_splits(mb_executor* ex, const mb_src& l, const mb_src& r, uint32_t tile_items,
                   uint64_t tiles, U flip, uint32_t* splits) {
-  const bool wide = l.len + r.len >= kSplitWideItems;
+  const bool wide = (l.len + r.len) * sizeof(U) >= kSplitWideBytes;
   const uint64_t threads = (tiles + 1) * (wide ? 2 : 8);
   auto kern = wide ? window_splits_kernel<U, ENC, 2> : window_splits_kernel<U, ENC, 8>;
   kern<<<(unsigned)((threads + kThreads - 1) / kThreads), kThreads, 0, ex->stream>>>(
