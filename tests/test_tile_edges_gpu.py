@@ -86,10 +86,9 @@ def test_small_sorts(ex, n, dtype, vdtype):
     perm = orc.radix_perm([k])
     dk = ex.to_device(k)
     if vdtype is None:
-        if np.dtype(dtype).kind == "f":
-            pytest.skip("keys alone sort through the comparator, which leaves NaN unspecified")
-        got = ex.to_host(vector.sort(ex, dk, op.Less))
-        np.testing.assert_array_equal(got, k[perm])
+        less = op.pred2("total_less" if np.dtype(dtype).kind == "f" else "less")
+        got = ex.to_host(vector.sort(ex, dk, less))
+        np.testing.assert_array_equal(got.view(np.uint8), k[perm].view(np.uint8))
         return
     v = seeded(vdtype, n, n + 1)
     sk, sv = vector.radix_sort_pairs(ex, dk, ex.to_device(v))
@@ -115,10 +114,10 @@ def test_small_sort_constant_keys_and_device_length(ex):
     np.testing.assert_array_equal(ex.to_host(sv), v[keep][perm])
 
 
-# Onesweep passes whose peers come half from ballots: a popular digit in some
-# passes only, partial last tiles, and 64-bit keys.
+# Onesweep passes some of whose peers come from ballots, as 64-bit keys always have it: a popular
+# digit in some passes only, partial last tiles.
 @pytest.mark.parametrize("n", [20000, 8192 * 5, 300_001])
-@pytest.mark.parametrize("dtype", [np.uint32, np.int32, np.float32, np.int64])
+@pytest.mark.parametrize("dtype", [np.int64, np.uint64, np.float64])
 def test_mixed_radix_rounds(ex, n, dtype):
     from massively_b200 import vector
     k = seeded(dtype, n, n)
@@ -132,6 +131,71 @@ def test_mixed_radix_rounds(ex, n, dtype):
     sk, sv = vector.radix_sort_pairs(ex, ex.to_device(k), ex.to_device(v))
     np.testing.assert_array_equal(ex.to_host(sv), v[perm])
     np.testing.assert_array_equal(ex.to_host(sk).view(np.uint8), k[perm].view(np.uint8))
+
+
+# 4-byte keys take ballots from 2^25 items (csrc/radix.cu kMixItems): a partial last tile, keys
+# over all digits, and few digits with many peers.
+@pytest.mark.parametrize("dtype", [np.uint32, np.int32, np.float32])
+@pytest.mark.parametrize("digits", ["all", "few"])
+def test_mixed_radix_rounds_of_long_columns(ex, dtype, digits):
+    import torch
+
+    from massively_b200 import vector
+    n = (1 << 25) + 4097
+    g = torch.Generator(device="cuda").manual_seed(5)
+    bits = torch.randint(-(1 << 31), 1 << 31, (n,), generator=g, device="cuda", dtype=torch.int32)
+    if digits == "few":
+        bits &= 0x01030007 - (1 << 31)
+    k = {"u": bits.view(torch.uint32), "i": bits, "f": bits.view(torch.float32)}[np.dtype(dtype).kind]
+    # the radix order as that of int32 numbers
+    enc = {"u": bits ^ -(1 << 31), "i": bits, "f": bits ^ ((bits >> 31) & 0x7FFFFFFF)}[
+        np.dtype(dtype).kind]
+    order = torch.sort(enc, stable=True).indices
+    v = ex.from_tensor(torch.arange(n, device="cuda", dtype=torch.int32))
+    sk, sv = vector.radix_sort_pairs(ex, ex.from_tensor(k), v)
+    ex.sync()
+    assert torch.equal(sv.tensor, order.to(torch.int32))
+    assert torch.equal(sk.tensor.view(torch.int32), bits[order])
+
+
+# Splits by two lanes (csrc/merge.cu kSplitWideBytes: 2^28 bytes of both lists) and the last size
+# that takes eight.
+@pytest.mark.parametrize("width", [4, 8])
+@pytest.mark.parametrize("past", [0, 1, 100_003])
+def test_merge_splits_of_long_lists(ex, width, past):
+    import torch
+
+    from massively_b200 import vector
+    t = torch.int32 if width == 4 else torch.int64
+    n = (1 << 28) // width - 1 + past
+    nl = n // 3
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x = torch.randint(-(1 << 30), 1 << 30, (n,), generator=g, device="cuda", dtype=t)
+    l, r = torch.sort(x[:nl]).values, torch.sort(x[nl:]).values
+    got = vector.merge(ex, ex.from_tensor(l), ex.from_tensor(r))
+    ex.sync()
+    assert torch.equal(got.tensor, torch.sort(x).values)
+
+
+# More tiles of a set operation than CTAs stay on the GPU at a time (6 per SM): CTAs take a second
+# tile into the same buffers.
+@pytest.mark.parametrize("dtype", [np.uint32, np.int64])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_set_windows_of_many_tiles(ex, dtype, shift):
+    import torch
+
+    from massively_b200 import vector
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    tile = 32768 // np.dtype(dtype).itemsize
+    nl, nr = 6 * sms * tile + 12_345, 4 * sms * tile + 1
+    lk, rk = _sorted(dtype, nl, 7, "less", nl), _sorted(dtype, nr, 8, "less", nl)
+    pad = np.zeros(shift, dtype)
+    l = ex.to_device(np.concatenate([pad, lk])).slice(shift)
+    r = ex.to_device(np.concatenate([pad, rk])).slice(shift)
+    np.testing.assert_array_equal(ex.to_host(vector.set_intersection(ex, l, r)),
+                                  orc.set_intersection(lk, rk, "less"))
+    np.testing.assert_array_equal(ex.to_host(vector.set_difference(ex, l, r)),
+                                  orc.set_difference(lk, rk, "less"))
 
 
 # The two-level look-back (csrc/lookback_group.cuh): more than 32 groups of 32
