@@ -64,7 +64,7 @@ def test_shipped_table_backs_the_database(tmp_path):
     # the package (device "*"); the caller's own record wins over it.
     path = str(tmp_path / "db.json")
     assert tune.lookup("NVIDIA B200", "radix", "u32/f32", 1 << 27, path) is None
-    assert tune.lookup("NVIDIA B200", "radix", "u32/f32", 1 << 27, path, shipped=True) == 9
+    assert tune.lookup("NVIDIA B200", "radix", "u32/f32", 1 << 27, path, shipped=True) == 6
     key = tune._key("NVIDIA B200", "radix", "u32/f32", 1 << 27)
     tune.save_db({key: {"config": 2, "ms": 1.0}}, path)
     assert tune.lookup("NVIDIA B200", "radix", "u32/f32", 1 << 27, path, shipped=True) == 2
