@@ -1,6 +1,7 @@
-// lookback.cuh -- tile status words and the warp-wide decoupled look-back
-// used by every single-pass kernel (scan, compaction, segmented scan and
-// reduce, by-key algorithms).
+// lookback.cuh -- tile status words of every single-pass kernel, and the
+// warp-wide decoupled look-back of the segmented and by-key kernels, set_union
+// and the float scans under MIN, MAX and MUL (the other scans, compaction and the
+// window set kernels: lookback_group.cuh, over the same words).
 //
 // A tile publishes its aggregate (flag 1) as soon as it has reduced its own
 // items, then its inclusive prefix (flag 2) once it knows its exclusive

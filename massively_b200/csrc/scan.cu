@@ -111,6 +111,10 @@ __device__ __forceinline__ void store_vec(T* p, uint64_t elem, const T (&src)[16
 template <class T, int OP>
 constexpr bool kTwoLevel = !std::is_floating_point<T>::value || OP == MB_OP_ADD;
 
+// The tile of configuration 0 (left_fold picks the same one at run time).
+template <class T, int OP>
+using LbCfg = std::conditional_t<kTwoLevel<T, OP>, SmemCfg<T>, BigCfg<T>>;
+
 template <class T, int OP, bool PACKED>
 __device__ __forceinline__ T scan_lookback(const TileState<T, PACKED>& st,
                                            const ScanParams<T>& p, uint64_t tile,
@@ -293,10 +297,10 @@ __device__ __forceinline__ void named_sync(int id, int count) {
 // bulk load lands and the eight compute warps scan their rows, so the
 // look-back's L2 round trips leave the tile's critical path: by the time the
 // tile's own aggregate is known its exclusive prefix usually is too.  The
-// compute warps publish the aggregate after phase 1 and the inclusive prefix
-// after joining the look-back warp.  (The look-back never needs the tile's
-// own aggregate; the fold order is the same as warp 0's, so float results
-// are unchanged.)
+// compute warps publish the aggregate after phase 1; under the left fold they
+// also publish the inclusive prefix after joining the look-back warp.  (The
+// look-back needs the tile's own aggregate only in the last tile of a group,
+// to publish the group's.)
 template <class T, int OP, bool PACKED, class C>
 __global__ void __launch_bounds__(kThreads + 32)
     scan_smem_lb_kernel(const T* __restrict__ in, T* __restrict__ out, uint64_t n,
@@ -355,15 +359,17 @@ __global__ void __launch_bounds__(kThreads + 32)
     const T excl = s_excl;
     bool h = tile > 0;
     T acc = excl;
-    T agg = s_wtot[0];
     for (int w = 0; w < kWarps; ++w) {
       s_pre[w] = acc;
       s_has[w] = h;
       acc = h ? op(acc, s_wtot[w]) : s_wtot[w];
       h = true;
-      if (w > 0) agg = op(agg, s_wtot[w]);
     }
-    if (!kTwoLevel<T, OP> && tile > 0) st.publish(tile, kFlagIncl, op(excl, agg));
+    if constexpr (!kTwoLevel<T, OP>) {
+      T agg = s_wtot[0];
+      for (int w = 1; w < kWarps; ++w) agg = op(agg, s_wtot[w]);
+      if (tile > 0) st.publish(tile, kFlagIncl, op(excl, agg));
+    }
   }
   named_sync(1, kThreads);
   smem_phase3<T, OP, C>(buf, tile, n, full, out, p, s_pre, s_has);
@@ -532,8 +538,8 @@ int scan_run(mb_executor* ex, const mb_src& in, int op, bool exclusive, const vo
   const bool smem_path = plain && in.len_dev == nullptr;
   int shape = smem_path ? std::max(0, ex->tune[MB_TUNE_SCAN]) : 0;
   if (smem_path && shape == 0 && left_fold<T>(op)) shape = 2;
-  // shapes: 0 = look-back warp, default tile; 1 = warp 0 runs the look-back,
-  // default tile; 2 = look-back warp, 64 KB tiles
+  // shapes: 0 = look-back warp, 32 KB tiles (64 KB under a left fold); 1 = warp
+  // 0 runs the look-back, 32 KB tiles; 2 = look-back warp, 64 KB tiles
   const uint64_t tile_items = !smem_path ? ScanCfg<T>::TILE
                               : shape == 2 ? BigCfg<T>::TILE : SmemCfg<T>::TILE;
   const uint64_t tiles = (cap + tile_items - 1) / tile_items;
@@ -573,13 +579,14 @@ int scan_run(mb_executor* ex, const mb_src& in, int op, bool exclusive, const vo
   } while (0)
 #define MB_SCAN_LAUNCH(OPID)                                                                    \
   do {                                                                                          \
+    using Lb = LbCfg<T, OPID>;                                                                  \
     if (smem_path) {                                                                            \
       if (shape == 1)                                                                           \
         MB_SCAN_SMEM(OPID, SmemCfg<T>);                                                         \
       else if (shape == 2)                                                                      \
         MB_SCAN_LB(OPID, BigCfg<T>);                                                            \
       else                                                                                      \
-        MB_SCAN_LB(OPID, SmemCfg<T>);                                                           \
+        MB_SCAN_LB(OPID, Lb);                                                                   \
     } else if (plain) {                                                                         \
       scan_kernel<T, OPID, true, PACKED><<<grid, block, 0, ex->stream>>>(s, out.data, cap, p, st); \
     } else {                                                                                    \
@@ -708,8 +715,7 @@ int scan_noalloc_run(mb_executor* ex, const mb_src& in, int op, const mb_col& ou
 #define MB_SCAN_NOALLOC_LAUNCH(OPID)                                                            \
   do {                                                                                          \
     if (smem_path) {                                                                            \
-      auto kern = big ? scan_smem_lb_kernel<T, OPID, PACKED, BigCfg<T>>                         \
-                      : scan_smem_lb_kernel<T, OPID, PACKED, SmemCfg<T>>;                       \
+      auto kern = scan_smem_lb_kernel<T, OPID, PACKED, LbCfg<T, OPID>>;                         \
       if (smem > 48 * 1024)                                                                     \
         MB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,         \
                                      (int)smem));                                               \

@@ -43,7 +43,9 @@ const char* mb_tune_describe(int family, int config) {
            "the source interval";
   if (config == 0) {
     switch (family) {
-      case MB_TUNE_SCAN: return "scan one 32 KB tile per CTA, a ninth warp runs the look-back";
+      case MB_TUNE_SCAN: 
+        return "scan one 32 KB tile per CTA (64 KB for float operators other than add), a ninth "
+               "warp runs the look-back";
       case MB_TUNE_REDUCE: return "reduce 256 threads x 4 x 16-byte vectors, fixed grid";
       case MB_TUNE_SELECT: return "compaction 256 threads x 16 items";
       default: break;
