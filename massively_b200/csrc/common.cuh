@@ -473,6 +473,19 @@ __device__ __forceinline__ U enc_bits(U raw) {
   }
 }
 
+// The bits that enc_bits encoded.
+template <class U, int ENC>
+__device__ __forceinline__ U dec_bits(U u) {
+  constexpr U sign = (U)1 << (sizeof(U) * 8 - 1);
+  if constexpr (ENC == kEncFloat) {
+    return (u & sign) ? (U)(u ^ sign) : (U)~u;
+  } else if constexpr (ENC == kEncSigned) {
+    return (U)(u ^ sign);
+  } else {
+    return u;
+  }
+}
+
 // Order-preserving radix encoding of massively/src/core/radix.rs:46-89:
 // unsigned as is, signed with the sign bit flipped, floats in total order
 // (negative: every bit inverted; otherwise the sign bit set).

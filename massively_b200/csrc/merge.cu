@@ -520,11 +520,7 @@ __device__ __forceinline__ U ord_of(U raw, U flip) {
 template <class U, int ENC>
 __device__ __forceinline__ U ord_to_raw(U u, U flip) {
   u ^= flip;
-  if constexpr (ENC == 2) {
-    constexpr U sign = (U)1 << (sizeof(U) * 8 - 1);
-    return (u & sign) ? (U)(u ^ sign) : (U)~u;
-  }
-  return u;
+  return ENC == 2 ? dec_bits<U, kEncFloat>(u) : u;
 }
 
 // The merge-path split of every tile boundary by groups of G lanes, G + 1

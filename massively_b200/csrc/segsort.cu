@@ -104,10 +104,7 @@ __device__ __forceinline__ uint32_t ss_encode(uint32_t raw, int desc, int ieee) 
 
 template <int ENC>
 __device__ __forceinline__ uint32_t ss_decode(uint32_t u, int desc) {
-  if (desc) u = ~u;
-  if constexpr (ENC == kEncFloat) return (u & 0x80000000u) ? (u ^ 0x80000000u) : ~u;
-  else if constexpr (ENC == kEncSigned) return u ^ 0x80000000u;
-  else return u;
+  return dec_bits<uint32_t, ENC>(desc ? ~u : u);
 }
 
 template <bool PLAIN>

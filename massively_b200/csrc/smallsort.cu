@@ -37,15 +37,13 @@ struct SmallSmem {
 
 template <class K>
 __device__ __forceinline__ K small_enc(K raw, int enc) {
-  constexpr K sign = (K)1 << (sizeof(K) * 8 - 1);
-  if (enc == kEncFloat) return (raw & sign) ? (K)~raw : (K)(raw ^ sign);
-  return enc == kEncSigned ? (K)(raw ^ sign) : raw;
+  if (enc == kEncFloat) return enc_bits<K, kEncFloat>(raw);
+  return enc == kEncSigned ? enc_bits<K, kEncSigned>(raw) : raw;
 }
 template <class K>
 __device__ __forceinline__ K small_dec(K u, int enc) {
-  constexpr K sign = (K)1 << (sizeof(K) * 8 - 1);
-  if (enc == kEncFloat) return (u & sign) ? (K)(u ^ sign) : (K)~u;
-  return enc == kEncSigned ? (K)(u ^ sign) : u;
+  if (enc == kEncFloat) return dec_bits<K, kEncFloat>(u);
+  return enc == kEncSigned ? dec_bits<K, kEncSigned>(u) : u;
 }
 
 template <class V, class K, int ITEMS>
